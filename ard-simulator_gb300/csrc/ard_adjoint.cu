@@ -30,6 +30,7 @@
 #include "ard_engine.h"
 #include "ard_gb300.h"
 #include "ard_kernels.cuh"
+#include "ard_modal.cuh"
 
 using namespace ard;
 
@@ -62,7 +63,7 @@ struct AdjBuffers {
 // Launch attributes of the kernels launched from this file.
 template <typename T>
 int configure_adjoint(Ctx* ctx) {
-  const int msmem = (int)(kModalSmemElems * sizeof(T));
+  const int msmem = (int)modal_smem_bytes<T>();
   ARD_CUDA(cudaFuncSetAttribute(modal_kernel<T, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, msmem));
   ARD_CUDA(cudaFuncSetAttribute(modal_kernel<T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, msmem));
   if (ctx->fused_faces) {
@@ -126,9 +127,10 @@ int launch_adjoint_step(Ctx* ctx, int t, int tstep, cudaStream_t s, cudaStream_t
     }
     ARD_CUDA(cudaGetLastError());
     ModalArgs<T> ma{buf, ctx->d_dct, ctx->d_tiles, (int)ctx->tiles.size(), ctx->d_srcpts, ctx->d_recpts,
-                    ctx->d_series, ctx->max_steps, ctx->d_tb, tstep, par, (const T*)ab.resid, ctx->n_rec_total};
-    const size_t msmem = kModalSmemElems * sizeof(T);
-    const int mgrid = grid_for((long long)ctx->tiles.size(), 1, ctx->num_sms * 2);
+                    ctx->d_series, ctx->max_steps, ctx->d_tb, tstep, par, (const T*)ab.resid, ctx->n_rec_total,
+                    ctx->d_modal_maps, ctx->d_err};
+    const size_t msmem = modal_smem_bytes<T>();
+    const int mgrid = grid_for((long long)ctx->tiles.size(), 1, ctx->num_sms * modal_blocks_per_sm<T>());
     if (ctx->arith == ARD_ARITH_REFERENCE)
       ARD_CUDA(launch_dep(modal_kernel<T, true, true>, mgrid, kModalThreads, msmem, s, ma));
     else

@@ -402,7 +402,7 @@ __global__ void srcgrad_kernel(const T* __restrict__ buf, const DctDev* __restri
   const PointDev q = srcs[r];
   const DctDev& D = dct[q.part];
   const int local = r - D.src0;
-  const int ntiles = D.nbx * D.nby * D.nbz;
+  const int ntiles = D.ntiles;
   T s = 0;
   for (int i = lane; i < ntiles; i += 32) s += buf[D.srcpart + (long long)i * D.nsrc + local];
   s = warp_sum(s);

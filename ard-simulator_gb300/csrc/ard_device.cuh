@@ -41,14 +41,19 @@
 namespace ard {
 
 constexpr int kMaxPointsPerPart = 8;  // sources or recorders per air partition
-constexpr int kModalThreads = 256;    // 8 warps per modal tile
+constexpr int kModalWarps = 4;        // warps of a modal tile's block
+constexpr int kModalThreads = 32 * kModalWarps;
+constexpr int kModalTX = 32, kModalTY = 32;   // kx and ky extent of a modal tile
+// Blocks of the modal kernel per SM (FP32: 164 registers, 61 KB of shared memory
+// each; FP64: 255 registers, 112 KB).
+template <typename T>
+constexpr int modal_blocks_per_sm() { return sizeof(T) == 4 ? 3 : 2; }
 constexpr int kMaxPmlLayers = 12;
 
 struct DctDev {
   int w, h, d, wp;
-  int G, rpc, kxt;         // lanes per ky row, ky rows per tile, kx per tile (4 G)
-  int nbx, nby, nbz, TZ;   // tiles along kx, ky, kz
-  int tile0;
+  int nbx, nby, nbz;       // modal tiles along kx, ky and (of each kz parity) kz
+  int tile0, ntiles;       // first modal tile, 2 nbx nby nbz of them
   int src0, nsrc;          // attached sources (PointDev table)
   int rec0, nrec;          // attached recorders
   long long M[2];
@@ -67,6 +72,17 @@ struct DctDev {
   double sf;               // forward scale 1 / (2 sqrt(2N))
   double si;               // inverse scale 1 / sqrt(2N)
   double damping;
+};
+
+// One tile of the modal update: 32 kx x 32 ky x the planes kz0, kz0 + 2, ..
+// (nkz of them, one kz parity) of an air partition.
+struct ModalTile {
+  int part;
+  int kx0, ky0, kz0;
+  int nkz;
+  int bx, by, bz;      // slabs of the contraction partials RX, RY, RZ
+  int local;           // index among the partition's tiles (point partials)
+  int pad[3];
 };
 
 struct PointDev {

@@ -20,6 +20,7 @@
 #include "ard_gb300.h"
 #include "ard_kernels.cuh"
 #include "ard_mma.cuh"
+#include "ard_modal.cuh"
 
 using namespace ard;
 
@@ -93,7 +94,7 @@ static int validate_scene(const ard_scene& s, std::string* err) {
 // translation unit holds its own instances of the kernel templates): the FP64
 // modal kernel needs more than 48 KB of dynamic shared memory.
 static int configure_kernels(Ctx* ctx) {
-  const int modal_smem = (int)(kModalSmemElems * elem_size(ctx));
+  const int modal_smem = (int)(ctx->prec == ARD_PREC_F64 ? modal_smem_bytes<double>() : modal_smem_bytes<float>());
   // The attribute belongs to the kernel, process-wide, not to the context:
   // set the device's opt-in maximum so that contexts with different layer
   // sizes can be interleaved in one process.
@@ -167,8 +168,7 @@ extern "C" int ard_create(const ard_scene* scenes, int32_t n_scenes, const ard_o
   ctx->smem_per_sm = prop.sharedMemPerMultiprocessor;
   const bool autotune = opt && opt->autotune != 0;
   auto describe = [](const Ctx* c) {
-    return std::string("tiles x") + std::to_string(c->tune_tiles) + ", lanes/row " +
-           (c->tune_g_shift == 0 ? "fit" : (c->tune_g_shift == 1 ? "narrow" : "narrower")) + ", faces " + (c->fused_faces ? "fused" : (c->mma_faces ? "tensor-core" : "gemm")) + ", " +
+    return std::string("tiles x") + std::to_string(c->tune_tiles) + ", faces " + (c->fused_faces ? "fused" : (c->mma_faces ? "tensor-core" : "gemm")) + ", " +
            std::to_string(c->tiles.size()) + " modal tiles, " + std::to_string(c->ngroups) + " air stream(s)";
   };
   if (!autotune) {
@@ -185,8 +185,8 @@ extern "C" int ard_create(const ard_scene* scenes, int32_t n_scenes, const ard_o
   }
   // Autotuner: build the context for each candidate layout, time real steps
   // (CUDA graphs, the production path), keep the fastest.
-  struct Cand { int tiles, gshift, gemm; };
-  const Cand cands[] = {{1, 2, 0}, {2, 2, 0}, {4, 2, 0}, {1, 1, 0}, {2, 1, 0}, {1, 0, 0}, {2, 0, 0}, {1, 2, 1}};
+  struct Cand { int tiles, gemm; };
+  const Cand cands[] = {{1, 0}, {2, 0}, {4, 0}, {1, 1}};
   std::unique_ptr<Ctx> best;
   float best_ms = 0.f;
   std::string report;
@@ -197,7 +197,7 @@ extern "C" int ard_create(const ard_scene* scenes, int32_t n_scenes, const ard_o
     c->use_graphs = ctx->use_graphs; c->device = ctx->device; c->arith = ctx->arith; c->adjoint = ctx->adjoint;
     c->debug_sync = ctx->debug_sync; c->num_sms = ctx->num_sms; c->smem_optin = ctx->smem_optin;
     c->smem_per_sm = ctx->smem_per_sm;
-    c->tune_tiles = cd.tiles; c->tune_g_shift = cd.gshift; c->tune_gemm = cd.gemm;
+    c->tune_tiles = cd.tiles; c->tune_gemm = cd.gemm;
     int rc = build_layout(c.get(), scenes, n_scenes);
     if (rc == ARD_OK) rc = configure_kernels(c.get());
     // the GEMM candidate is a distinct layout only where the fused transforms fit
@@ -348,7 +348,7 @@ int launch_step(Ctx* ctx, int par, int tstep, cudaStream_t s, cudaStream_t s2, b
   if (int rc = launch_pml<T>(ctx, par, tstep, sp)) return rc;
   if (!ctx->dct.empty()) {
     const int gx = ctx->num_sms * 4;
-    const size_t msmem = kModalSmemElems * sizeof(T);
+    const size_t msmem = modal_smem_bytes<T>();
     // one stage of one group's air branch on stream `st`
     auto stage = [&](int k, const Ctx::AirGroup& G, cudaStream_t st) -> int {
       if (k == kStageFwdRows) {
@@ -372,8 +372,9 @@ int launch_step(Ctx* ctx, int par, int tstep, cudaStream_t s, cudaStream_t s2, b
         const int n = G.t_hi - G.t_lo;
         if (n > 0) {
           ModalArgs<T> ma{buf, ctx->d_dct, ctx->d_tiles + G.t_lo, n, ctx->d_srcpts, ctx->d_recpts,
-                          ctx->d_series, ctx->max_steps, ctx->d_t, tstep, par, nullptr, 0};
-          const int mgrid = grid_for(n, 1, ctx->num_sms * 2);
+                          ctx->d_series, ctx->max_steps, ctx->d_t, tstep, par, nullptr, 0,
+                          ctx->d_modal_maps, ctx->d_err};
+          const int mgrid = grid_for(n, 1, ctx->num_sms * modal_blocks_per_sm<T>());
           if (ctx->arith == ARD_ARITH_REFERENCE)
             ARD_CUDA(launch_dep(modal_kernel<T, true, false>, mgrid, kModalThreads, msmem, st, ma));
           else

@@ -69,7 +69,7 @@ struct Ctx {
   std::vector<unsigned char> masks;
   std::vector<int> cell_iface;              // interface of every face cell
   std::vector<PointDev> srcpts, recpts;
-  std::vector<int4> tiles;
+  std::vector<ModalTile> tiles;
   JobList fwd1, fwd2, inv1, inv2;           // two-pass GEMM face transforms
   std::vector<Face2DJob> fwd2d, inv2d;      // fused face transforms
   std::vector<SumJob> psum;                 // partial sums before the inverse transforms
@@ -111,7 +111,6 @@ struct Ctx {
   bool adjoint = false;
   // layout choices (the autotuner varies them; defaults are the heuristics)
   int tune_tiles = 1;      // modal tiles per wave slot (x 2 per SM): kz split finer when > 1
-  int tune_g_shift = 2;    // k > 0: ky rows k lane-sizes narrower (more kx tiles, more ky rows per tile)
   int tune_gemm = 0;       // 1: two-pass GEMM face transforms even when the fused ones fit
   std::string tuning;      // description of the chosen layout
   // adjoint face transforms (options.adjoint): fused 2D jobs and the two-pass
@@ -136,7 +135,7 @@ struct Ctx {
   int* d_cell_iface = nullptr;
   PointDev* d_srcpts = nullptr;
   PointDev* d_recpts = nullptr;
-  int4* d_tiles = nullptr;
+  ModalTile* d_tiles = nullptr;
   XformJob *d_fwd1 = nullptr, *d_fwd2 = nullptr, *d_inv1 = nullptr, *d_inv2 = nullptr;
   Face2DJob *d_fwd2d = nullptr, *d_inv2d = nullptr;
   SumJob* d_psum = nullptr;
@@ -149,7 +148,9 @@ struct Ctx {
   void* d_phist = nullptr;        // PmlHist<T> read by the PML kernel (adjoint contexts only)
   MmaJob* d_mjobs[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   int* d_err = nullptr;           // set by a kernel whose bounded wait ran out (checked on synchronize)
-  CUtensorMap* d_pml_maps = nullptr;   // tensor maps of the PML tile loads (build_pml_maps)
+  CUtensorMap* d_maps = nullptr;       // all tensor maps (build_tensor_maps), then the parts:
+  CUtensorMap* d_modal_maps = nullptr; // modal plane loads
+  CUtensorMap* d_pml_maps = nullptr;   // PML tile loads
   CUtensorMap* d_pml_amaps = nullptr;  // the adjoint PML kernel's (options.adjoint)
 
   // neighbourhood recording (ard_record_neighbourhoods): the 10 x 10 x 10
@@ -171,7 +172,7 @@ enum { kStagePml = 0, kStageFwdRows, kStageFwdCols, kStageModal, kStageRecorder,
        kStageIface, kNumStages };
 
 int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes);
-int build_pml_maps(Ctx* ctx);
+int build_tensor_maps(Ctx* ctx);
 int build_pml_hist_maps(Ctx* ctx, const void* hist, long long hlen, long long slots, CUtensorMap** out);
 cudaError_t launch_mma(Ctx* ctx, int k, cudaStream_t s);
 void free_ctx_device(Ctx* ctx);

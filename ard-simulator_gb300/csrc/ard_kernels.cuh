@@ -7,8 +7,8 @@
 //                       air partition, fused per layer pair in shared memory
 //                       (face_gemm_kernel: the same as two GEMM passes where
 //                       a layer pair does not fit)
-//   modal_kernel        F = expansion of the face transforms (+ point
-//                       sources); M(t) = a (2 cos M(t-1) - M(t-2) + psi F);
+//   modal_kernel        (ard_modal.cuh) F = expansion of the face transforms
+//                       (+ point sources); M(t) = a (2 cos M(t-1) - M(t-2) + psi F);
 //                       contraction of M(t) onto the face rows and the
 //                       recorder cells
 //   post_modal_kernel   recorder samples of step t + sums of the contraction
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(256) post_modal_kernel(PostModalArgs<T> a) {
     const PointDev q = a.recs[r];
     const DctDev& D = a.dct[q.part];
     const int local_r = r - D.rec0;
-    const int ntiles = D.nbx * D.nby * D.nbz;
+    const int ntiles = D.ntiles;
     T s = 0;
     for (int i = lane; i < ntiles; i += 32) s += a.buf[D.recpart + (long long)i * D.nrec + local_r];
     s = warp_sum(s);
@@ -960,416 +960,6 @@ inline cudaError_t launch_face2d(bool split, long long n, int max_ctas, size_t s
   const long long b = std::max(1LL, std::min(2 * n, (long long)max_ctas));
   return launch_dep(face2d_kernel<T>, b, kFace2DThreads, smem, s, buf, jobs, (int)n, sm);
 }
-
-// ---------------------------------------------------------------------------
-// Modal update
-// ---------------------------------------------------------------------------
-
-template <typename T>
-struct ModalArgs {
-  T* buf;
-  const DctDev* dct;
-  const int4* tiles;        // {air partition, kx tile, ky tile, kz tile}
-  int ntiles;
-  const PointDev* srcs;
-  const PointDev* recs;
-  const float* series;      // [n_sources][max_steps]
-  long long max_steps;
-  const long long* tcount;  // steps completed before the current launch sequence
-  int tstep;                // step offset inside the sequence (adjoint: counted backwards)
-  int par;
-  const T* resid;           // adjoint: recorder residuals [steps][n_rec_total]
-  int n_rec_total;
-};
-
-// Shared memory of the modal kernel, in elements of T: the ky-contraction
-// slots, point coefficients, recorder reduction, and the double-buffered
-// per-plane inputs (7 four-element rows per thread + 6 PX values per ky row).
-constexpr int kModalRySlot = 3 * 1024;  // [3 n][rpc * kxt = 1024]
-constexpr int kModalStageCz = 7 * 4 * kModalThreads + 32 * 6;   // [8 warps][4]: Cd row kz, n = 0..2
-constexpr int kModalStage = kModalStageCz + 32;
-constexpr int kModalSmemElems =
-    2 * kModalRySlot + 2 * kMaxPointsPerPart * 128 + 8 * kMaxPointsPerPart + 2 * kModalStage;
-
-// One block (8 warps) per tile of kxt kx x rpc ky x TZ kz modes; a thread
-// owns 4 consecutive kx of one ky row.  Per mode it reads M(t-1), M(t-2)
-// and the two tables and writes M(t) (all 128-bit, row pitch wp), expands
-// the face transforms into the force mode F, and contracts M(t) onto the face
-// rows: along kx by a shuffle butterfly (partial per kx tile), along ky
-// through shared memory (partial per ky tile), along kz in registers
-// (partial per kz tile).  REF selects the reference's arithmetic.
-//
-// ADJ runs the transposed step of the adjoint, backwards in time, on the
-// adjoint modal levels mu: mu(t) = alpha mu(t+1) - a mu(t+2) + G(t), where
-// alpha and -a are the forward recurrence's coefficients of M(t-1) and M(t-2)
-// and G is the expansion of the adjoint face transforms with the REDFT01
-// weights plus the recorder residuals injected with the recorder basis.  The
-// contraction then runs on beta mu(t) (beta: the forward coefficient of the
-// force mode F) with the REDFT10 weights onto the face rows and onto the
-// source cells (source-series gradient partials).
-template <typename T, bool REF, bool ADJ = false>
-__global__ void __launch_bounds__(kModalThreads, 2) modal_kernel(ModalArgs<T> a) {
-  grid_dependency_wait();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* ry_s = reinterpret_cast<T*>(smem_raw);
-  T* cws = ry_s + 2 * kModalRySlot;                  // [kMaxPointsPerPart][128]
-  T* cwr = cws + kMaxPointsPerPart * 128;            // [kMaxPointsPerPart][128]
-  T* red = cwr + kMaxPointsPerPart * 128;            // [8 warps][kMaxPointsPerPart]
-  T* stage = red + 8 * kMaxPointsPerPart;            // [2][kModalStage]
-  __shared__ int pts_y[2][kMaxPointsPerPart], pts_z[2][kMaxPointsPerPart];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  T* __restrict__ buf = a.buf;
-  const long long t = ADJ ? (*a.tcount - a.tstep) : (*a.tcount + a.tstep);
-
-  for (int tile_id = blockIdx.x; tile_id < a.ntiles; tile_id += gridDim.x) {
-    const int4 tl = a.tiles[tile_id];
-    const DctDev& D = a.dct[tl.x];
-    const int w = D.w, h = D.h, d = D.d, wp = D.wp, G = D.G, KXT = D.kxt, RPC = D.rpc;
-    const int rs = warp * (32 / G) + lane / G;   // row slot in the tile
-    const int li = lane % G;
-    const int kl0 = 4 * li;
-    const int kx0 = tl.y * KXT + kl0;
-    const int ky0 = tl.z * RPC;
-    const int ky = ky0 + rs;
-    const bool rowok = ky < h;
-    const bool lanok = rowok && kx0 < wp;
-    const int kz0 = tl.w * D.TZ, kz1 = min(kz0 + D.TZ, d);
-    const int nsrc = D.nsrc, nrec = D.nrec;
-    const T* Cw = buf + D.cw;
-    const T* Ch = buf + D.ch;
-    const T* Cd = buf + D.cd;
-    const T* Cwi = Cw + (long long)w * w;
-    const T* Chi = Ch + (long long)h * h;
-    const T* Cdi = Cd + (long long)d * d;
-    // injected points (sources; adjoint: recorders) and read-out points
-    // (recorders; adjoint: sources) with their bases
-    const int ninj = ADJ ? nrec : nsrc, nout = ADJ ? nsrc : nrec;
-    const PointDev* injp = ADJ ? a.recs + D.rec0 : a.srcs + D.src0;
-    const PointDev* outp = ADJ ? a.srcs + D.src0 : a.recs + D.rec0;
-    const T* Iw = ADJ ? Cwi : Cw;
-    const T* Ih = ADJ ? Chi : Ch;
-    const T* Id = ADJ ? Cdi : Cd;
-    const T* Ow = ADJ ? Cw : Cwi;
-    const T* Oh = ADJ ? Ch : Chi;
-    const T* Od = ADJ ? Cd : Cdi;
-
-    __syncthreads();  // the previous tile is done with shared memory
-    for (int i = tid; i < ninj * KXT; i += kModalThreads) {
-      const int s = i / KXT, kl = i - s * KXT, kx = tl.y * KXT + kl;
-      const PointDev q = injp[s];
-      if constexpr (ADJ) {
-        const T v = a.resid[t * a.n_rec_total + q.slot];
-        cws[s * 128 + kl] = kx < w ? (T)D.si * v * Iw[(long long)kx * w + q.x] : (T)0;
-      } else {
-        const float v = (t < a.max_steps) ? a.series[(long long)q.slot * a.max_steps + t] : 0.0f;
-        cws[s * 128 + kl] = kx < w ? (T)D.sf * (T)v * Iw[(long long)kx * w + q.x] : (T)0;
-      }
-      if (kl == 0) { pts_y[0][s] = q.y; pts_z[0][s] = q.z; }
-    }
-    for (int i = tid; i < nout * KXT; i += kModalThreads) {
-      const int r = i / KXT, kl = i - r * KXT, kx = tl.y * KXT + kl;
-      const PointDev q = outp[r];
-      cwr[r * 128 + kl] = kx < w ? Ow[(long long)kx * w + q.x] : (T)0;
-      if (kl == 0) { pts_y[1][r] = q.y; pts_z[1][r] = q.z; }
-    }
-    __syncthreads();
-
-    T cx[4][3];
-    bool act[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      act[e] = rowok && (kx0 + e < w);
-      const int kxe = min(kx0 + e, w - 1);
-#pragma unroll
-      for (int n = 0; n < 3; ++n) cx[e][n] = Cw[(long long)kxe * w + n];
-    }
-    const T wx0 = (kx0 == 0) ? (T)0.5 : (T)1;   // REDFT01 halves the k = 0 row
-    const int kyc = rowok ? ky : 0;
-    T cy[3];
-#pragma unroll
-    for (int n = 0; n < 3; ++n) cy[n] = Ch[(long long)kyc * h + n];
-    const T wy = (ky == 0) ? (T)0.5 : (T)1;
-    // the REDFT01 halving of the k = 0 rows sits in the contraction (forward)
-    // or in the expansion (adjoint)
-    const T wxc = ADJ ? (T)1 : wx0, wyc = ADJ ? (T)1 : wy;
-    const int pyr = ky & 1;
-    const long long planeX = (long long)d * h, planeY = (long long)d * wp, planeZ = (long long)h * wp;
-    const T* PX = buf + D.PX;
-    const T* PYr = buf + D.PY + pyr * 3 * planeY;
-    T pz[2][3][4], rz[2][3][4];
-#pragma unroll
-    for (int pm = 0; pm < 2; ++pm)
-#pragma unroll
-      for (int n = 0; n < 3; ++n) {
-        if (lanok) {
-          load4(buf + D.PZ + (pm * 3 + n) * planeZ + (long long)ky * wp + kx0, pz[pm][n]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) pz[pm][n][e] = 0;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) rz[pm][n][e] = 0;
-      }
-    T racc[kMaxPointsPerPart];
-#pragma unroll
-    for (int r = 0; r < kMaxPointsPerPart; ++r) racc[r] = 0;
-    const T* Mcur = buf + (ADJ ? D.AM[a.par ^ 1] : D.M[a.par ^ 1]);   // M(t-1) (adjoint: mu(t+1))
-    T* Mout = buf + (ADJ ? D.AM[a.par] : D.M[a.par]);                 // M(t-2) -> M(t) (adjoint: mu(t+2) -> mu(t))
-    const T* tabA = buf + D.tabA;
-    const T* tabB = buf + D.tabB;
-    const T damping = (T)D.damping;
-
-    // ky contraction.  A warp holds rpw = 32 / G ky rows; with G = 8 the rows
-    // r and r + 2 (same parity) are folded by one shuffle, so every warp leaves
-    // rfold <= 2 partial rows in the slot, at [(warp rfold + row) 3 + n][kxt].
-    // Rows past h carry zeros (their modes are masked).  The parity of a
-    // partial row is (warp rpw + row) & 1 (ky0 is even).  Reducers: one
-    // thread per (parity pm, n, kx quad) sums the warps' partials of parity pm
-    // (start (pm 3 + n) kxt + 4 kq, stride 6 kxt: 8 terms, or 4 when a warp
-    // holds a single row and only every other warp has parity pm).
-    const int rpw = 32 / G;
-    const int rfold = rpw < 2 ? rpw : 2;
-    const int yrow = lane / G;                       // row within the warp
-    const bool ywrite = yrow < rfold;
-    const int yslot = (warp * rfold + (ywrite ? yrow : 0)) * 3 * KXT + kl0;
-    const int nquad = KXT / 4;
-    const int yterms = rfold == 2 ? 8 : 4;
-    int ysrc = -1;
-    T* ydst = buf;
-    if (tid < 6 * nquad) {
-      const int pm = tid / (3 * nquad);
-      const int rem = tid - pm * 3 * nquad;
-      const int n = rem / nquad, kq = rem - n * nquad;
-      const int kx = tl.y * KXT + 4 * kq;
-      if (kx < wp) {
-        ysrc = (pm * 3 + n) * KXT + 4 * kq;
-        ydst = buf + D.RY + ((long long)tl.z * 6 + pm * 3 + n) * planeY + kx;
-      }
-    }
-    // kx contraction output of this lane (after the reduce-scatter below):
-    // q = parity 3 + n for lanes whose low bits below G / 8 are zero
-    const int xq = li / (G >> 3);
-    const bool xwrite = rowok && (li & ((G >> 3) - 1)) == 0 && xq < 6;
-    T* const xdst = buf + D.RX + ((long long)tl.y * 6 + (xwrite ? xq : 0)) * planeX + (rowok ? ky : 0);
-
-    // per-plane inputs of plane kz into stage buffer sb (asynchronous)
-    auto issue = [&](int kz, int sb) {
-      T* st = stage + sb * kModalStage;
-      const long long row = ((long long)kz * h + (rowok ? ky : 0)) * wp + (lanok ? kx0 : 0);
-      cp_async4(st + (0 * kModalThreads + tid) * 4, Mcur + row, lanok);
-      cp_async4(st + (1 * kModalThreads + tid) * 4, Mout + row, lanok);
-      cp_async4(st + (2 * kModalThreads + tid) * 4, tabA + row, lanok);
-      cp_async4(st + (3 * kModalThreads + tid) * 4, tabB + row, lanok);
-#pragma unroll
-      for (int n = 0; n < 3; ++n)
-        cp_async4(st + ((4 + n) * kModalThreads + tid) * 4,
-                  PYr + n * planeY + (long long)kz * wp + (lanok ? kx0 : 0), lanok);
-      if (li < 6) {
-        const int pm = li / 3, n = li - pm * 3;
-        cp_async_scalar(st + 7 * 4 * kModalThreads + rs * 6 + li,
-                        PX + (pm * 3 + n) * planeX + (long long)kz * h + (rowok ? ky : 0), rowok);
-      }
-      if (lane < 3) cp_async_scalar(st + kModalStageCz + warp * 4 + lane, Cd + (long long)kz * d + lane, true);
-    };
-
-    auto body = [&](auto parity, int kz, int sb) {
-      constexpr int PZ = decltype(parity)::value;  // kz & 1 (kz0 is even)
-      const T* st = stage + sb * kModalStage;
-      T cz[3];
-#pragma unroll
-      for (int n = 0; n < 3; ++n) cz[n] = st[kModalStageCz + warp * 4 + n];
-      const T wz = (kz == 0) ? (T)0.5 : (T)1;
-      const T wzc = ADJ ? (T)1 : wz;
-      T px[2][3];
-#pragma unroll
-      for (int pm = 0; pm < 2; ++pm)
-#pragma unroll
-        for (int n = 0; n < 3; ++n) px[pm][n] = st[7 * 4 * kModalThreads + rs * 6 + pm * 3 + n];
-      T py[3][4];
-      T m[4], mp[4], ta[4], tb[4];
-      const long long row = ((long long)kz * h + ky) * wp + kx0;
-      load4(st + (0 * kModalThreads + tid) * 4, m);
-      load4(st + (1 * kModalThreads + tid) * 4, mp);
-      load4(st + (2 * kModalThreads + tid) * 4, ta);
-      load4(st + (3 * kModalThreads + tid) * 4, tb);
-#pragma unroll
-      for (int n = 0; n < 3; ++n) load4(st + ((4 + n) * kModalThreads + tid) * 4, py[n]);
-      if (!lanok) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) tb[e] = 1;  // keeps the reference arithmetic finite on idle lanes
-      }
-      T F[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if constexpr (ADJ) {
-          T fx = 0, fy = 0, fz = 0;
-#pragma unroll
-          for (int n = 0; n < 3; ++n) {
-            fx += cx[e][n] * px[e & 1][n];
-            fy += cy[n] * py[n][e];
-            fz += cz[n] * pz[PZ][n][e];
-          }
-          F[e] = (e == 0 ? wx0 : (T)1) * fx + wy * fy + wz * fz;
-        } else {
-          T f = 0;
-#pragma unroll
-          for (int n = 0; n < 3; ++n) f += cx[e][n] * px[e & 1][n];
-#pragma unroll
-          for (int n = 0; n < 3; ++n) f += cy[n] * py[n][e];
-#pragma unroll
-          for (int n = 0; n < 3; ++n) f += cz[n] * pz[PZ][n][e];
-          F[e] = f;
-        }
-      }
-      for (int s = 0; s < ninj; ++s) {
-        const T coef = Ih[(long long)kyc * h + pts_y[0][s]] * Id[(long long)kz * d + pts_z[0][s]];
-        T c[4];
-        load4(cws + s * 128 + kl0, c);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) F[e] += c[e] * coef;
-      }
-      T Mn[4];
-      if constexpr (ADJ) {
-        T beta[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          T v;
-          if (REF) {
-            v = damping * ((T)2 * m[e] * ta[e] - mp[e]) + F[e];
-            beta[e] = damping * ((T)2 / tb[e]) * ((T)1 - ta[e]);
-          } else {
-            v = damping * (((T)2 * m[e] - mp[e]) - (T)2 * ta[e] * m[e]) + F[e];
-            beta[e] = damping * tb[e];
-          }
-          Mn[e] = act[e] ? v : (T)0;
-        }
-        if (lanok) store4(Mout + row, Mn);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) Mn[e] *= beta[e];   // contracted: the adjoint of the force mode
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          T v;
-          if (REF)  // dct_partition.cpp:68: a (2 M cwt - M_prev + (2 F / w2) (1 - cwt))
-            v = damping * ((T)2 * m[e] * ta[e] - mp[e] + ((T)2 * F[e] / tb[e]) * ((T)1 - ta[e]));
-          else      // the same recurrence with ta = 1 - cwt, tb = 2 (1 - cwt) / w2
-            v = damping * (((T)2 * m[e] - mp[e]) - (T)2 * ta[e] * m[e] + tb[e] * F[e]);
-          Mn[e] = act[e] ? v : (T)0;
-        }
-        if (lanok) store4(Mout + row, Mn);
-      }
-      // contraction along kz (registers) and ky (folded partial rows in the slot)
-      T* slot = ry_s + PZ * kModalRySlot;
-      {
-        T ry[3][4];
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            rz[PZ][n][e] += wzc * cz[n] * Mn[e];
-            ry[n][e] = wyc * cy[n] * Mn[e];
-          }
-        if (rfold == 2 && rpw == 4) {
-#pragma unroll
-          for (int n = 0; n < 3; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) ry[n][e] += __shfl_xor_sync(0xffffffffu, ry[n][e], 16);
-        }
-        if (ywrite) {
-#pragma unroll
-          for (int n = 0; n < 3; ++n) store4(slot + yslot + n * KXT, ry[n]);
-        }
-      }
-      // contraction along kx: even / odd kx sums v[q], q = parity 3 + n (two
-      // zero pads), then a reduce-scatter over the row's G lanes: three
-      // halving exchanges leave lane li with q = li / (G / 8), completed by a
-      // butterfly over the G / 8 lanes that share it
-      {
-        T v[8];
-#pragma unroll
-        for (int n = 0; n < 3; ++n) {
-          v[n] = wxc * cx[0][n] * Mn[0] + cx[2][n] * Mn[2];
-          v[3 + n] = cx[1][n] * Mn[1] + cx[3][n] * Mn[3];
-        }
-        v[6] = 0;
-        v[7] = 0;
-        const int o4 = G >> 1, o2 = G >> 2, o1 = G >> 3;
-        const bool u4 = (li & o4) != 0, u2 = (li & o2) != 0, u1 = (li & o1) != 0;
-        T h4[4], h2[2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          h4[i] = (u4 ? v[4 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, u4 ? v[i] : v[4 + i], o4);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-          h2[i] = (u2 ? h4[2 + i] : h4[i]) + __shfl_xor_sync(0xffffffffu, u2 ? h4[i] : h4[2 + i], o2);
-        T h1 = (u1 ? h2[1] : h2[0]) + __shfl_xor_sync(0xffffffffu, u1 ? h2[0] : h2[1], o1);
-        for (int o = o1 >> 1; o > 0; o >>= 1) h1 += __shfl_xor_sync(0xffffffffu, h1, o);
-        if (xwrite) xdst[(long long)kz * h] = h1;
-      }
-      for (int r = 0; r < nout; ++r) {
-        const T coef = Oh[(long long)kyc * h + pts_y[1][r]] * Od[(long long)kz * d + pts_z[1][r]];
-        T c[4];
-        load4(cwr + r * 128 + kl0, c);
-        racc[r] += coef * (c[0] * Mn[0] + c[1] * Mn[1] + c[2] * Mn[2] + c[3] * Mn[3]);
-      }
-      __syncthreads();
-      // ky contraction of this kz: sums of the warps' partial rows of parity pm
-      if (ysrc >= 0) {
-        T sum[4] = {0, 0, 0, 0};
-        for (int k = 0; k < yterms; ++k) {
-          T p4[4];
-          load4(slot + ysrc + k * 6 * KXT, p4);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) sum[e] += p4[e];
-        }
-        store4(ydst + (long long)kz * wp, sum);
-      }
-    };
-
-    // software pipeline: plane kz+1 loads while plane kz computes
-    issue(kz0, 0);
-    cp_async_commit();
-    for (int kz = kz0; kz < kz1; kz += 2) {
-      if (kz + 1 < kz1) issue(kz + 1, 1);
-      cp_async_commit();
-      cp_async_wait<1>();
-      __syncwarp();
-      body(std::integral_constant<int, 0>{}, kz, 0);
-      if (kz + 1 < kz1) {
-        if (kz + 2 < kz1) issue(kz + 2, 0);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncwarp();
-        body(std::integral_constant<int, 1>{}, kz + 1, 1);
-      }
-    }
-    cp_async_wait<0>();
-    if (lanok) {
-#pragma unroll
-      for (int pm = 0; pm < 2; ++pm)
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
-          store4(buf + D.RZ + ((long long)tl.w * 6 + pm * 3 + n) * planeZ + (long long)ky * wp + kx0, rz[pm][n]);
-    }
-    if (nout > 0) {
-#pragma unroll
-      for (int r = 0; r < kMaxPointsPerPart; ++r) {
-        if (r < nout) {
-          const T s = warp_sum(racc[r]);
-          if (lane == 0) red[warp * kMaxPointsPerPart + r] = s;
-        }
-      }
-      __syncthreads();
-      if (tid < nout) {
-        T s = 0;
-        for (int k = 0; k < kModalThreads / 32; ++k) s += red[k * kMaxPointsPerPart + tid];
-        const int local = (tl.y * D.nby + tl.z) * D.nbz + tl.w;
-        buf[(ADJ ? D.srcpart : D.recpart) + (long long)local * nout + tid] = s;
-      }
-    }
-  }
-}
-
 
 // ---------------------------------------------------------------------------
 // PML

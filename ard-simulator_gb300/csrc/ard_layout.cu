@@ -19,6 +19,7 @@
 #include "ard_gb300.h"
 #include "ard_kernels.cuh"
 #include "ard_mma.cuh"
+#include "ard_modal.cuh"
 
 using namespace ard;
 
@@ -492,50 +493,54 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     ctx->recpts.insert(ctx->recpts.end(), recs_of[k].begin(), recs_of[k].end());
   }
 
-  // ---- modal tiling ----
-  // A tile is 8 warps; a thread owns 4 consecutive kx.  G lanes cover one ky
-  // row (G = 8, 16 or 32, the smallest with 4 G >= min(wp, 128)), so a tile
-  // spans kxt = 4 G kx and rpc = 256 / G ky rows.  The kz extent TZ (even, or
-  // the whole depth) is chosen so that the tiles fill the GPU at least twice.
-  long long col_tiles = 0;
-  for (DctDev& D : ctx->dct) {
-    const int need = std::min(D.wp, 128) / 4;
-    D.G = need <= 8 ? 8 : (need <= 16 ? 16 : 32);
-    for (int k = 0; k < ctx->tune_g_shift && D.G > 8; ++k) D.G /= 2;
-    D.kxt = 4 * D.G;
-    D.rpc = kModalThreads / D.G;
-    D.nbx = (D.wp + D.kxt - 1) / D.kxt;
-    D.nby = (D.h + D.rpc - 1) / D.rpc;
-    col_tiles += (long long)D.nbx * D.nby;
-  }
-  // resident slots: 2 tiles per SM.  kz splits: as many as still fit one
-  // wave, then more while that evens out the last wave (the blocks take the
-  // tiles round-robin, so a last wave that is half full costs a whole tile
-  // time: c4's 749 full-depth columns are 2.46 waves of 304 slots, split in
-  // two they are 4.93)
-  const long long slots = (long long)ctx->num_sms * 2 * std::max(1, ctx->tune_tiles);
-  long long nbz_all = col_tiles > 0 ? std::max(1LL, slots / col_tiles) : 1;
-  if (col_tiles > 0) {
-    auto wave_eff = [&](long long nb) {
-      const long long T = col_tiles * nb, waves = (T + slots - 1) / slots;
-      return (double)T / (double)(waves * slots);
+  // ---- modal tiling (ModalTile) ----
+  // Planes per tile: a tile costs its planes and about three and a half more
+  // (descriptors, first loads, its part of three Z layers read, written and
+  // summed), and the blocks take the tiles in waves of the resident slots.
+  // GB300, modal + sums: 100^3 cells 24.0 us at 4 planes (one wave), 27.6 at 2,
+  // 26.0 at 8, 65 at 50; 232 x 178 x 300 cells 88 us at 38 (one wave), 96 at 8,
+  // 124 at 75 (slots left empty).  In FP64 the planes' arithmetic outweighs
+  // the rest (60 x 60 x 40 and four smaller: 50 us at 1 plane, 56 at 2, 78 at 3).
+  {
+    const int per_sm = ctx->prec == ARD_PREC_F64 ? modal_blocks_per_sm<double>() : modal_blocks_per_sm<float>();
+    const long long slots = (long long)ctx->num_sms * per_sm * std::max(1, ctx->tune_tiles);
+    auto count = [&](int tz) {
+      long long c = 0;
+      for (const DctDev& D : ctx->dct)
+        c += 2LL * ((D.wp + kModalTX - 1) / kModalTX) * ((D.h + kModalTY - 1) / kModalTY) * (((D.d + 1) / 2 + tz - 1) / tz);
+      return c;
     };
-    const long long base = nbz_all;
-    double best = wave_eff(base);
-    for (long long nb = base + 1; nb <= 4 * base + 4; ++nb)
-      if (wave_eff(nb) > best + 0.03) { best = wave_eff(nb); nbz_all = nb; }
-  }
-  for (size_t k = 0; k < ctx->dct.size(); ++k) {
-    DctDev& D = ctx->dct[k];
-    long long nbz = std::max(1LL, std::min<long long>(nbz_all, D.d / 2));
-    int TZ = (int)((D.d + nbz - 1) / nbz);
-    if (TZ < D.d) TZ += TZ & 1;  // even, so every kz tile starts on an even plane
-    D.TZ = TZ;
-    D.nbz = (D.d + D.TZ - 1) / D.TZ;
-    D.tile0 = (int)ctx->tiles.size();
-    for (int bx = 0; bx < D.nbx; ++bx)
-      for (int by = 0; by < D.nby; ++by)
-        for (int bz = 0; bz < D.nbz; ++bz) ctx->tiles.push_back(make_int4((int)k, bx, by, bz));
+    const int least = ctx->prec == ARD_PREC_F64 ? 1 : 2;
+    int tz = least;
+    double best = 0;
+    for (int k = least; k <= 64; ++k) {
+      const double waves = (double)count(k) / (double)slots;
+      const double cost = ctx->prec == ARD_PREC_F64 ? (waves + 0.5) * (k + 0.5)
+                                                    : (waves > 6 ? waves + 0.5 : std::ceil(waves)) * (k + 3.5);
+      if (k == least || cost < best) { best = cost; tz = k; }
+    }
+    for (size_t k = 0; k < ctx->dct.size(); ++k) {
+      DctDev& D = ctx->dct[k];
+      const int planes = (D.d + 1) / 2;   // of the even parity; the odd one has D.d / 2
+      D.nbx = (D.wp + kModalTX - 1) / kModalTX;
+      D.nby = (D.h + kModalTY - 1) / kModalTY;
+      D.nbz = (planes + tz - 1) / tz;
+      D.tile0 = (int)ctx->tiles.size();
+      for (int bz = 0; bz < D.nbz; ++bz)
+        for (int par = 0; par < 2; ++par)
+          for (int by = 0; by < D.nby; ++by)
+            for (int bx = 0; bx < D.nbx; ++bx) {
+              ModalTile t{};
+              t.part = (int)k;
+              t.kx0 = bx * kModalTX; t.ky0 = by * kModalTY; t.kz0 = 2 * bz * tz + par;
+              // an odd parity one plane short may leave its last tile empty: only the zero RZ partials are written
+              t.nkz = std::max(0, std::min(tz, (par ? D.d / 2 : planes) - bz * tz));
+              t.bx = bx; t.by = by; t.bz = bz;
+              t.local = (int)ctx->tiles.size() - D.tile0;
+              ctx->tiles.push_back(t);
+            }
+      D.ntiles = (int)ctx->tiles.size() - D.tile0;
+    }
   }
 
   // ---- state block: everything a checkpoint holds, contiguous ----
@@ -545,6 +550,10 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
   auto set_faces = [](DctDev& D, long long base, long long* fx, long long* fy, long long* fz) {
     *fx = base; *fy = base + 6LL * D.d * D.h; *fz = *fy + 6LL * D.d * D.wp;
   };
+  // the modal tables just before the modal levels: the four arrays of a
+  // partition lie one array region apart (one tensor map, build_tensor_maps)
+  for (DctDev& D : ctx->dct) D.tabA = pool.take((long long)D.wp * D.h * D.d);
+  for (DctDev& D : ctx->dct) D.tabB = pool.take((long long)D.wp * D.h * D.d);
   ctx->state_begin = pool.off;
   for (DctDev& D : ctx->dct) D.M[0] = pool.take((long long)D.wp * D.h * D.d);
   for (DctDev& D : ctx->dct) D.M[1] = pool.take((long long)D.wp * D.h * D.d);
@@ -588,8 +597,6 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
 
   // ---- constants and per-step scratch ----
   for (DctDev& D : ctx->dct) {
-    const long long Np = (long long)D.wp * D.h * D.d;
-    D.tabA = pool.take(Np); D.tabB = pool.take(Np);
     D.cw = cos_table(D.w); D.ch = cos_table(D.h); D.cd = cos_table(D.d);
     const long long FX = 6LL * D.d * D.h, FY = 6LL * D.d * D.wp, FZ = 6LL * D.h * D.wp;
     set_faces(D, pool.take(faces(D)), &D.pX, &D.pY, &D.pZ);
@@ -601,8 +608,8 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     D.tmpX = pool.take(std::max(FX, 6LL * D.h * dp));
     D.tmpY = pool.take(std::max(FY, 6LL * D.w * dp));
     D.tmpZ = pool.take(std::max(FZ, 6LL * D.w * hp));
-    D.recpart = pool.take(std::max(1, D.nrec) * (long long)D.nbx * D.nby * D.nbz);
-    D.srcpart = pool.take(std::max(1, D.nsrc) * (long long)D.nbx * D.nby * D.nbz);
+    D.recpart = pool.take(std::max(1, D.nrec) * (long long)D.ntiles);
+    D.srcpart = pool.take(std::max(1, D.nsrc) * (long long)D.ntiles);
   }
 
   // ---- dense-transform scratch (initial pressure, field readout): 3 x the largest air partition ----
@@ -1050,7 +1057,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     if (ctx->mma_faces && !ctx->mjobs[k].empty() && (rc = up(&ctx->d_mjobs[k], ctx->mjobs[k]))) return rc;
   ARD_CUDA(cudaMalloc(&ctx->d_err, sizeof(int)));
   ARD_CUDA(cudaMemset(ctx->d_err, 0, sizeof(int)));
-  if (int rc = build_pml_maps(ctx)) return rc;
+  if (int rc = build_tensor_maps(ctx)) return rc;
   if (ctx->adjoint) {
     if ((rc = up(&ctx->d_adj1_2d, ctx->adj1_2d))) return rc;
     if ((rc = up(&ctx->d_adj2_2d, ctx->adj2_2d))) return rc;
@@ -1118,7 +1125,7 @@ void free_ctx_device(Ctx* ctx) {
                   ctx->d_adjg[2], ctx->d_adjg[3], ctx->d_tb, ctx->d_phist, ctx->d_psum,
                   ctx->d_cell_iface, ctx->d_mjobs[0], ctx->d_mjobs[1], ctx->d_mjobs[2], ctx->d_mjobs[3],
                   ctx->d_mjobs[4], ctx->d_mjobs[5], ctx->d_mjobs[6], ctx->d_mjobs[7],
-                  ctx->d_err, ctx->d_pml_maps, ctx->d_pml_amaps};
+                  ctx->d_err, ctx->d_maps};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
@@ -1146,63 +1153,103 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
+// A tensor of `rank` dimensions (innermost first; strides[k] the elements
+// between neighbours along dimension k + 1) at `base`, read in boxes of `box`.
+// Elements outside the tensor read as zero.
+static int encode_map(Ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
+                      const long long* strides, const cuuint32_t* box) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (!enc) { ctx->err = "cuTensorMapEncodeTiled is not available from the driver"; return ARD_ERR_CUDA; }
+  const size_t es = elem_size(ctx);
+  const CUtensorMapDataType type =
+      ctx->prec == ARD_PREC_F64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  cuuint64_t bytes[4] = {0, 0, 0, 0};
+  for (int k = 0; k + 1 < rank; ++k) bytes[k] = (cuuint64_t)strides[k] * es;
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUresult r = enc(map, type, rank, const_cast<void*>(base), dims, bytes, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    ctx->err = "cuTensorMapEncodeTiled failed (error " + std::to_string((int)r) + ")";
+    return ARD_ERR_CUDA;
+  }
+  return ARD_OK;
+}
+
 // One PML slab field as a [L][A][B] tensor (row pitch Bp) at `base`, or with
 // `slots` > 0 as [slots][L][A][B] with `slot_stride` elements between slots,
 // read in boxes of box_b x box_a (x 1 x 1).  Elements outside the tensor read
 // as zero, the reference's sentinel.
 static int encode_slab_map(Ctx* ctx, CUtensorMap* map, const PmlDev& P, const void* base, cuuint32_t box_b,
                            cuuint32_t box_a, long long slots = 0, long long slot_stride = 0) {
-  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-  if (!enc) { ctx->err = "cuTensorMapEncodeTiled is not available from the driver"; return ARD_ERR_CUDA; }
-  const size_t es = elem_size(ctx);
-  const CUtensorMapDataType type =
-      ctx->prec == ARD_PREC_F64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  const cuuint32_t rank = slots > 0 ? 4 : 3;
   const cuuint64_t dims[4] = {(cuuint64_t)P.B, (cuuint64_t)P.A, (cuuint64_t)P.L, (cuuint64_t)std::max(1LL, slots)};
-  const cuuint64_t strides[3] = {(cuuint64_t)P.Bp * es, (cuuint64_t)P.A * P.Bp * es, (cuuint64_t)slot_stride * es};
+  const long long strides[3] = {P.Bp, (long long)P.A * P.Bp, slot_stride};
   const cuuint32_t box[4] = {box_b, box_a, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = enc(map, type, rank, const_cast<void*>(base), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    ctx->err = "cuTensorMapEncodeTiled failed for a PML slab (error " + std::to_string((int)r) + ")";
-    return ARD_ERR_CUDA;
-  }
-  return ARD_OK;
+  return encode_map(ctx, map, base, slots > 0 ? 4 : 3, dims, strides, box);
 }
 
-// The tensor maps of the PML kernels' tile loads, with the box of the tile
-// each one feeds (PmlStage, PmlAdjStage): per slab p (halo 3, x from b0 - 4),
-// phi_a (halo 2 along a) and phi_b (halo 2 along b, x from b0 - 4) of both
-// time levels; with the adjoint also its three levels of p and two of each
-// phi.
-int build_pml_maps(Ctx* ctx) {
-  if (ctx->pml.empty()) return ARD_OK;
+// The tensor maps of a context, in one device buffer:
+//  - the modal kernel's plane loads (kModalMaps per air partition): the tables
+//    and modal levels as [4 or 2][d][h][wp] in boxes of one 32 x 32 plane tile
+//    of each array, the transformed Y layers as [6][d][wp] in boxes of one
+//    plane's 32 kx of all six;
+//  - the PML kernels' tile loads, with the box of the tile each one feeds
+//    (PmlStage, PmlAdjStage): per slab p (halo 3, x from b0 - 4), phi_a (halo
+//    2 along a) and phi_b (halo 2 along b, x from b0 - 4) of both time levels;
+//    with the adjoint also its three levels of p and two of each phi.
+int build_tensor_maps(Ctx* ctx) {
   const size_t es = elem_size(ctx);
-  const cuuint32_t PW = kPmlTB + 8;
   char* base = (char*)ctx->d_buf;
-  std::vector<CUtensorMap> maps(6 * ctx->pml.size()), amaps(ctx->adjoint ? 7 * ctx->pml.size() : 0);
+  const size_t n_modal = kModalMaps * ctx->dct.size(), n_pml = 6 * ctx->pml.size(),
+               n_adj = ctx->adjoint ? 7 * ctx->pml.size() : 0;
+  std::vector<CUtensorMap> maps(n_modal + n_pml + n_adj);
+  if (maps.empty()) return ARD_OK;
+  for (size_t k = 0; k < ctx->dct.size(); ++k) {
+    const DctDev& D = ctx->dct[k];
+    CUtensorMap* m = &maps[kModalMaps * k];
+    const long long apart = D.tabB - D.tabA;
+    if (D.M[0] - D.tabB != apart || D.M[1] - D.M[0] != apart || (ctx->adjoint && D.AM[1] - D.AM[0] != apart)) {
+      ctx->err = "internal: modal arrays out of step";
+      return ARD_ERR_STATE;
+    }
+    auto arrays = [&](CUtensorMap* map, long long first, int count) {
+      const cuuint64_t dims[4] = {(cuuint64_t)D.wp, (cuuint64_t)D.h, (cuuint64_t)D.d, (cuuint64_t)count};
+      const long long strides[3] = {D.wp, (long long)D.h * D.wp, apart};
+      const cuuint32_t box[4] = {kModalTX, kModalTY, 1, (cuuint32_t)count};
+      return encode_map(ctx, map, base + first * es, 4, dims, strides, box);
+    };
+    if (int rc = arrays(m + kMapForward, D.tabA, 4)) return rc;
+    const cuuint64_t ydims[3] = {(cuuint64_t)D.wp, (cuuint64_t)D.d, 6};
+    const long long ystrides[2] = {D.wp, (long long)D.d * D.wp};
+    const cuuint32_t ybox[3] = {kModalTX, 1, 6};
+    if (int rc = encode_map(ctx, m + kMapPY, base + D.PY * es, 3, ydims, ystrides, ybox)) return rc;
+    if (ctx->adjoint) {
+      if (int rc = arrays(m + kMapTables, D.tabA, 2)) return rc;
+      if (int rc = arrays(m + kMapAdjoint, D.AM[0], 2)) return rc;
+    }
+  }
+  const cuuint32_t PW = kPmlTB + 8;
+  const cuuint32_t bb[3] = {PW, (cuuint32_t)kPmlTB, PW}, ba[3] = {kPmlTA + 6, kPmlTA + 4, kPmlTA};
   for (size_t k = 0; k < ctx->pml.size(); ++k) {
     const PmlDev& P = ctx->pml[k];
     const long long offs[6] = {P.p[0], P.p[1], P.pha[0], P.pha[1], P.phb[0], P.phb[1]};
-    const cuuint32_t bb[3] = {PW, (cuuint32_t)kPmlTB, PW}, ba[3] = {kPmlTA + 6, kPmlTA + 4, kPmlTA};
     for (int q = 0; q < 6; ++q)
-      if (int rc = encode_slab_map(ctx, &maps[6 * k + q], P, base + offs[q] * es, bb[q / 2], ba[q / 2])) return rc;
+      if (int rc = encode_slab_map(ctx, &maps[n_modal + 6 * k + q], P, base + offs[q] * es, bb[q / 2], ba[q / 2]))
+        return rc;
     if (ctx->adjoint) {
       const long long aoffs[7] = {P.ap[0], P.ap[1], P.ap[2], P.apha[0], P.apha[1], P.aphb[0], P.aphb[1]};
       const int kind[7] = {0, 0, 0, 1, 1, 2, 2};
       for (int q = 0; q < 7; ++q)
-        if (int rc = encode_slab_map(ctx, &amaps[7 * k + q], P, base + aoffs[q] * es, bb[kind[q]], ba[kind[q]]))
+        if (int rc = encode_slab_map(ctx, &maps[n_modal + n_pml + 7 * k + q], P, base + aoffs[q] * es, bb[kind[q]],
+                                     ba[kind[q]]))
           return rc;
     }
   }
-  ARD_CUDA(cudaMalloc(&ctx->d_pml_maps, sizeof(CUtensorMap) * maps.size()));
-  ARD_CUDA(cudaMemcpy(ctx->d_pml_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
-  if (ctx->adjoint) {
-    ARD_CUDA(cudaMalloc(&ctx->d_pml_amaps, sizeof(CUtensorMap) * amaps.size()));
-    ARD_CUDA(cudaMemcpy(ctx->d_pml_amaps, amaps.data(), sizeof(CUtensorMap) * amaps.size(), cudaMemcpyHostToDevice));
-  }
+  ARD_CUDA(cudaMalloc(&ctx->d_maps, sizeof(CUtensorMap) * maps.size()));
+  ARD_CUDA(cudaMemcpy(ctx->d_maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
+  ctx->d_modal_maps = ctx->d_maps;
+  ctx->d_pml_maps = ctx->d_maps + n_modal;
+  ctx->d_pml_amaps = ctx->d_maps + n_modal + n_pml;
   return ARD_OK;
 }
 
