@@ -68,8 +68,8 @@ int configure_adjoint(Ctx* ctx) {
   ARD_CUDA(cudaFuncSetAttribute(modal_kernel<T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, msmem));
   if (ctx->fused_faces) {
     const int f2d = std::max(ctx->smem_optin, (int)ctx->f2d_bytes);
-    ARD_CUDA(cudaFuncSetAttribute(face2d_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
-    ARD_CUDA(cudaFuncSetAttribute(face2d_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
+    ARD_CUDA(cudaFuncSetAttribute(face_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
+    ARD_CUDA(cudaFuncSetAttribute(face_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
   }
   ARD_CUDA(configure_face_gemm<T>());
   return ARD_OK;
@@ -115,8 +115,8 @@ int launch_adjoint_step(Ctx* ctx, int t, int tstep, cudaStream_t s, cudaStream_t
   if (!ctx->dct.empty()) {
     const int gx = ctx->num_sms * 4;
     if (ctx->fused_faces) {
-      ARD_CUDA(launch_face2d<T>(ctx->adj1_split, (long long)ctx->adj1_2d.size() / 2, gx, ctx->f2d_bytes, s, buf,
-                                ctx->d_adj1_2d, ctx->f2d_smem));
+      ARD_CUDA((launch_face<T, false>((long long)ctx->adj1_2d.size() / 2, gx, ctx->f2d_bytes, s, buf, ctx->d_adj1_2d,
+                                      ctx->f2d_smem)));
     } else if (ctx->mma_faces) {
       ARD_CUDA(launch_mma(ctx, 4, s));
       ARD_CUDA(launch_mma(ctx, 5, s));
@@ -144,8 +144,8 @@ int launch_adjoint_step(Ctx* ctx, int t, int tstep, cudaStream_t s, cudaStream_t
     }
     if (int rc2 = launch_post_modal<T>(ctx, s, 0, false)) return rc2;
     if (ctx->fused_faces) {
-      ARD_CUDA(launch_face2d<T>(ctx->adj2_split, (long long)ctx->adj2_2d.size() / 2, gx, ctx->f2d_bytes, s, buf,
-                                ctx->d_adj2_2d, ctx->f2d_smem));
+      ARD_CUDA((launch_face<T, true>((long long)ctx->adj2_2d.size() / 2, gx, ctx->f2d_bytes, s, buf, ctx->d_adj2_2d,
+                                     ctx->f2d_smem)));
     } else if (ctx->mma_faces) {
       ARD_CUDA(launch_mma(ctx, 6, s));
       ARD_CUDA(launch_mma(ctx, 7, s));

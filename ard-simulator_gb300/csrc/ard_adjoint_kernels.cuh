@@ -9,11 +9,11 @@
 //   pml_adjoint_kernel     transposed Grote-Sim update; accumulates the
 //                          gradient of every damping layer zeta(l) from the
 //                          forward PML history
-//   face2d / GEMM jobs     adjoint of the inverse face transform
+//   face / GEMM jobs       adjoint of the inverse face transform
 //   modal_kernel<ADJ>      transposed modal recurrence, recorder residual
 //                          injection, source-series gradient partials
 //   srcgrad_kernel         source-series gradient of step t
-//   face2d / GEMM jobs     adjoint of the forward face transform -> adjoint
+//   face / GEMM jobs       adjoint of the forward face transform -> adjoint
 //                          shell force of step t - 1
 #pragma once
 

@@ -162,13 +162,11 @@ struct XformJob {
   double scale;
 };
 
-// One fused 2D transform of a pair of face layers, for output columns
-// [u0, u0 + ub):
+// One fused 2D transform of a pair of face layers (ard_face.cuh), for a slab
+// of at most 32 output columns [u0, u0 + ub):
 //   out0 = scale A (X0 + X1) B,   out1 = scale A (X0 - X1) B
-// X0, X1: V x U, row pitch ld; A: V x V, B: U x U (row-contiguous copies
-// of the transform matrices, restricted to the slab's columns for B).
-// Forward: A = C_V, B(j, u) = C_U[u][j]; inverse: A(o, r) = Ci_V[r][o],
-// B(j, u) = Ci_U[j][u].
+// X0, X1: V x U, row pitch ld.  tabA, tabB: the parity-split tables of V and U
+// that the job's direction takes (forward: Hr, Hf; inverse: Hf, Hr).
 struct Face2DJob {
   long long in0, in1;
   long long out0, out1;
@@ -176,8 +174,8 @@ struct Face2DJob {
   int V, U, ld;
   int u0, ub;
   int which;     // 0: both outputs; 1: out0 only; 2: out1 only (a pair split over two blocks)
-  int narrow;    // 1: at most 16 columns (16 rows per warp)
-  int split;     // 1: the rows are split between the two CTAs of the cluster
+  int narrow;    // 1: at most 16 columns
+  int split;     // 1: the slab's work is halved between the two entries of the job (face_shape)
   int part;      // air partition (engine index)
   double scale;
 };

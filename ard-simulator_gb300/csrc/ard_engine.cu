@@ -103,15 +103,15 @@ static int configure_kernels(Ctx* ctx) {
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     if (ctx->fused_faces) {
-      ARD_CUDA(cudaFuncSetAttribute(face2d_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
-      ARD_CUDA(cudaFuncSetAttribute(face2d_cluster_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
+      ARD_CUDA(cudaFuncSetAttribute(face_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
+      ARD_CUDA(cudaFuncSetAttribute(face_kernel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
     }
   } else {
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     if (ctx->fused_faces) {
-      ARD_CUDA(cudaFuncSetAttribute(face2d_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
-      ARD_CUDA(cudaFuncSetAttribute(face2d_cluster_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
+      ARD_CUDA(cudaFuncSetAttribute(face_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
+      ARD_CUDA(cudaFuncSetAttribute(face_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
     }
   }
   ARD_CUDA(ctx->prec == ARD_PREC_F64 ? configure_face_gemm<double>() : configure_face_gemm<float>());
@@ -354,8 +354,7 @@ int launch_step(Ctx* ctx, int par, int tstep, cudaStream_t s, cudaStream_t s2, b
       if (k == kStageFwdRows) {
         if (ctx->fused_faces) {
           const int n = G.f_hi - G.f_lo;
-          ARD_CUDA(launch_face2d<T>(G.f_split, n, gx, ctx->f2d_bytes, st, buf, ctx->d_fwd2d + 2 * G.f_lo,
-                                    ctx->f2d_smem));
+          ARD_CUDA((launch_face<T, false>(n, gx, ctx->f2d_bytes, st, buf, ctx->d_fwd2d + 2 * G.f_lo, ctx->f2d_smem)));
         } else if (ctx->mma_faces) {
           ARD_CUDA(launch_mma(ctx, 0, st));
         } else {
@@ -387,8 +386,7 @@ int launch_step(Ctx* ctx, int par, int tstep, cudaStream_t s, cudaStream_t s2, b
       } else if (k == kStageInvCols) {
         if (ctx->fused_faces) {
           const int n = G.i_hi - G.i_lo;
-          ARD_CUDA(launch_face2d<T>(G.i_split, n, gx, ctx->f2d_bytes, st, buf, ctx->d_inv2d + 2 * G.i_lo,
-                                    ctx->f2d_smem));
+          ARD_CUDA((launch_face<T, true>(n, gx, ctx->f2d_bytes, st, buf, ctx->d_inv2d + 2 * G.i_lo, ctx->f2d_smem)));
         } else if (ctx->mma_faces) {
           ARD_CUDA(launch_mma(ctx, 2, st));
         } else {

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "ard_device.cuh"
+#include "ard_face.cuh"
 #include "ard_gb300.h"
 #include "ard_kernels.cuh"
 
@@ -81,7 +82,6 @@ struct Ctx {
   struct AirGroup {
     int part_lo = 0, part_hi = 0;
     int f_lo = 0, f_hi = 0, i_lo = 0, i_hi = 0;
-    bool f_split = false, i_split = false;   // the range holds row-split face jobs (cluster launch)
     int t_lo = 0, t_hi = 0, r_lo = 0, r_hi = 0, s_lo = 0, s_hi = 0;
     long long s_first = 0, s_total = 0;
   };
@@ -95,8 +95,9 @@ struct Ctx {
   std::vector<MmaJob> mjobs[8];            // forward pass 1, 2; inverse pass 1, 2; adjoint passes 1 .. 4
   int mtiles[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   std::vector<std::pair<int, long long>> mma_tables;   // extent -> offset of Chi, Clo, CiThi, CiTlo
-  Face2DSmem f2d_smem{0, 0, 0, 0};
+  FaceSmem f2d_smem{0, 0, 0, 0};
   size_t f2d_bytes = 0;
+  std::vector<std::pair<int, long long>> face_tables;  // extent -> offset of its parity-split tables
   std::vector<std::pair<int, long long>> cos_tables;  // extent -> offset
   long long n_pml_cells = 0, n_face_cells = 0;
   long long n_air_cells = 0;
@@ -116,7 +117,6 @@ struct Ctx {
   // adjoint face transforms (options.adjoint): fused 2D jobs and the two-pass
   // GEMM form (q rows, q columns, R columns, R rows)
   std::vector<Face2DJob> adj1_2d, adj2_2d;
-  bool adj1_split = false, adj2_split = false;
   JobList adjg[4];
   long long q_begin = 0, q_end = 0;          // adjoint face pressure (zeroed every adjoint step)
   bool adj_valid = false;                    // adjoint levels hold mu(0), mu(1) of the last ard_adjoint

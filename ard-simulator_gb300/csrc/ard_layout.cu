@@ -138,24 +138,21 @@ int zero_state(Ctx* ctx) {
   return ARD_OK;
 }
 
-// Balances the face jobs of one launch and pairs them for the two CTAs of a
-// cluster.  While the launch still fits in one wave of `slots` CTAs (it then
-// lasts as long as its largest job), the largest job is split: a two-output
-// job into one job per output (the same staging, half the arithmetic), then
-// a one-output job's rows between the two CTAs of its cluster (half the
-// staging and arithmetic each, the halves of T exchanged through distributed
-// shared memory).  A launch of many waves keeps whole jobs, two to a cluster,
-// one per CTA.  A 16-column job costs its warps as much as a 32-column one
-// (16 rows per warp instead of 8), so column splits would not shorten the
-// launch and are not made.  Output: pairs (jobs[2 i], jobs[2 i + 1]) for the
-// cluster of item i, largest first: a split job twice, or two whole jobs (the
-// last one padded by an empty job).  Returns whether any job's rows are split
-// (the launch then runs in clusters; without, one CTA per entry).
+// Balances the face jobs of one launch and pairs them.  While the launch still
+// fits in one wave of `slots` blocks (it then lasts as long as its largest
+// job), the largest job is split: a two-output job into one job per output,
+// then a one-output job into two halves (face_shape: one parity each, or half
+// of the columns each).  A launch of many waves keeps whole jobs, which read
+// their layers once for all their outputs.  The work model counts whole row
+// blocks of a warp, so a 16-column job weighs as much as a 32-column one.
+// Output: pairs (jobs[2 i], jobs[2 i + 1]), largest first: a split job twice,
+// or two whole jobs (the last one padded by an empty job).  Returns whether
+// any job is split.
 bool balance_face_jobs(std::vector<Face2DJob>* jobs, int slots) {
   // the arithmetic of one warp of a CTA of the job: rows of the warp's row
   // blocks x the slab's columns x both contractions, for one or two outputs
   auto work = [](const Face2DJob& j) {
-    const int rows = j.narrow ? 16 : 8, per_block = rows * kFace2DWarps;
+    const int rows = j.narrow ? 16 : 8, per_block = rows * (kFaceThreads / 32);
     const int nr = j.split ? (j.V + 1) / 2 : j.V;
     return (long long)((nr + per_block - 1) / per_block) * rows * (j.narrow ? 16 : 32) * (j.U + j.V) *
            (j.which == 0 ? 2 : 1);
@@ -214,6 +211,13 @@ bool balance_face_jobs(std::vector<Face2DJob>* jobs, int slots) {
   return split;
 }
 
+// Parity-split table `kind` (kFaceC / kFaceCi + kFaceHr / kFaceHf) of extent n.
+static long long face_table(const Ctx* ctx, int n, int kind) {
+  for (const auto& kv : ctx->face_tables)
+    if (kv.first == n) return kv.second + kind * face_table_elems(n);
+  return -1;
+}
+
 // Face transforms of the adjoint step, the transposes of the forward ones:
 //   adjoint of the inverse transform: Q[pm][n] = s_i Ci_V (q_n +/- q_{5-n}) Ci_U^T
 //     (the adjoint face pressure q -> the P arrays read by the adjoint modal step)
@@ -235,24 +239,25 @@ void build_adjoint_jobs(Ctx* ctx) {
     for (const Ax& a : axes) {
       const long long LS = (long long)a.V * a.ld;
       const long long UU = (long long)a.U * a.U, VV = (long long)a.V * a.V;
-      for (int u0 = 0; u0 < a.U; u0 += 32) {
+      for (int u0 = 0; ctx->fused_faces && u0 < a.U; u0 += 32) {
         const int ub = std::min(32, a.U - u0);
         for (int n = 0; n < 3; ++n) {
           Face2DJob j{};   // q layers n, 5-n -> P[0][n], P[1][n]
           j.in0 = a.q + n * LS; j.in1 = a.q + (5 - n) * LS;
           j.out0 = a.P + n * LS; j.out1 = a.P + (3 + n) * LS;
-          j.tabA = a.cV + VV; j.tabB = a.cU + 3 * UU;   // Ci_V, Ci_U^T
+          j.tabA = face_table(ctx, a.V, kFaceCi + kFaceHr); j.tabB = face_table(ctx, a.U, kFaceCi + kFaceHf);
           j.V = a.V; j.U = a.U; j.ld = a.ld; j.u0 = u0; j.ub = ub; j.scale = D.si;
           ctx->adj1_2d.push_back(j);
           Face2DJob k{};   // summed partials R[n], R[3+n] -> adjoint force layers n, 5-n
           k.in0 = a.R + n * LS; k.in1 = a.R + (3 + n) * LS;
           k.out0 = a.a + n * LS; k.out1 = a.a + (5 - n) * LS;
-          k.tabA = a.cV + 2 * VV; k.tabB = a.cU;          // C_V^T, C_U
+          k.tabA = face_table(ctx, a.V, kFaceC + kFaceHf); k.tabB = face_table(ctx, a.U, kFaceC + kFaceHr);
           k.V = a.V; k.U = a.U; k.ld = a.ld; k.u0 = u0; k.ub = ub; k.scale = D.sf;
           ctx->adj2_2d.push_back(k);
         }
       }
       // two-pass GEMM form (partitions whose layers do not fit in shared memory)
+      if (ctx->fused_faces || ctx->mma_faces) continue;
       for (int pm = 0; pm < 2; ++pm)
         for (int n = 0; n < 3; ++n) {
           XformJob j{};   // rows along U with Ci_U: A(o, j) = Ci_U[o][j]
@@ -815,7 +820,65 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     }
   }
 
-  // ---- transform jobs (GEMMs over the face layers) ----
+  // ---- fused face transforms (one kernel per direction) where a whole layer
+  // pair, both tables' columns and the intermediates fit 200 KB of shared
+  // memory: FP32 extents up to about 132 (larger faces have the rows to feed
+  // the tensor-core passes) ----
+  {
+    long long xs = 0, bs = 0;
+    auto pitch = [](int n) { const int n4 = (n + 3) & ~3; return n4 + ((n4 & 7) ? 8 : 4); };
+    auto axis = [&](int V, int U) {
+      xs = std::max(xs, (long long)V * std::max(pitch(U), pitch(V)));
+      bs = std::max(bs, 32LL * (((U + 3) & ~3) + 2 * ((V + 3) & ~3)));
+    };
+    for (const DctDev& D : ctx->dct) { axis(D.d, D.h); axis(D.d, D.w); axis(D.h, D.w); }
+    ctx->f2d_bytes = (size_t)(2 * xs + bs) * elem_size(ctx);
+    ctx->fused_faces = !ctx->dct.empty() && !ctx->tune_gemm &&
+                       ctx->f2d_bytes <= (size_t)std::min(ctx->smem_optin, 200 * 1024);
+  }
+  if (ctx->fused_faces) {
+    std::map<int, long long> tabs;
+    for (const DctDev& D : ctx->dct)
+      for (int n : {D.w, D.h, D.d})
+        if (!tabs.count(n)) tabs[n] = pool.take(4 * face_table_elems(n));
+    ctx->face_tables.assign(tabs.begin(), tabs.end());
+    for (size_t pi = 0; pi < ctx->dct.size(); ++pi) {
+      const DctDev& D = ctx->dct[pi];
+      struct Ax { long long f, p, P, R; int U, V, ld; };
+      const Ax axes[3] = {{D.fX, D.pX, D.PX, D.RX, D.h, D.d, D.h},
+                          {D.fY, D.pY, D.PY, D.RY, D.w, D.d, D.wp},
+                          {D.fZ, D.pZ, D.PZ, D.RZ, D.w, D.h, D.wp}};
+      for (const Ax& a : axes) {
+        const long long LS = (long long)a.V * a.ld;
+        for (int u0 = 0; u0 < a.U; u0 += 32) {
+          const int ub = std::min(32, a.U - u0);
+          for (int n = 0; n < 3; ++n) {
+            // forward: layers n, 5-n -> even / odd parts P[0][n], P[1][n]
+            Face2DJob j{};
+            j.in0 = a.f + n * LS; j.in1 = a.f + (5 - n) * LS;
+            j.out0 = a.P + n * LS; j.out1 = a.P + (3 + n) * LS;
+            j.tabA = face_table(ctx, a.V, kFaceC + kFaceHr); j.tabB = face_table(ctx, a.U, kFaceC + kFaceHf);
+            j.V = a.V; j.U = a.U; j.ld = a.ld; j.u0 = u0; j.ub = ub; j.scale = D.sf; j.part = (int)pi;
+            ctx->fwd2d.push_back(j);
+            // inverse: even / odd parts (partials summed beforehand) -> layers n, 5-n
+            Face2DJob k{};
+            k.in0 = a.R + n * LS; k.in1 = a.R + (3 + n) * LS;
+            k.out0 = a.p + n * LS; k.out1 = a.p + (5 - n) * LS;
+            k.tabA = face_table(ctx, a.V, kFaceCi + kFaceHf); k.tabB = face_table(ctx, a.U, kFaceCi + kFaceHr);
+            k.V = a.V; k.U = a.U; k.ld = a.ld; k.u0 = u0; k.ub = ub; k.scale = D.si; k.part = (int)pi;
+            ctx->inv2d.push_back(k);
+          }
+        }
+      }
+    }
+  }
+  // ---- tensor-core face transforms (FP32, two-pass form; ARD_FACE_MMA=0 keeps the CUDA-core passes) ----
+  {
+    const char* env = std::getenv("ARD_FACE_MMA");
+    ctx->mma_faces = ctx->prec == ARD_PREC_F32 && !ctx->fused_faces && !ctx->dct.empty() && !(env && env[0] == '0');
+    if (ctx->mma_faces) build_mma_jobs(ctx, [&](long long n) { return pool.take(n); });
+  }
+  // ---- CUDA-core GEMM jobs over the face layers (two-pass faces off the tensor cores) ----
   auto add_job = [](JobList& list, XformJob j) {
     const int Md = j.rows ? j.batch : j.n, Nd = j.rows ? j.n : j.batch;
     j.tn = (Nd + 63) / 64;
@@ -823,6 +886,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     list.add(j, j.ntiles);
   };
   for (const DctDev& D : ctx->dct) {
+    if (ctx->fused_faces || ctx->mma_faces) break;
     // layer [V][ld], transforms along U (fast) and V (slow)
     struct Axis { long long f, p, P, R, tmp; int nU, nV, ld; long long cU, cV; int nb; };
     const Axis axes[3] = {
@@ -862,50 +926,6 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     }
   }
 
-  // ---- fused face transforms (one kernel per direction) when a layer fits in shared memory ----
-  {
-    const size_t es0 = elem_size(ctx);
-    long long xs = 0, x1 = 0, bs = 0, ts = 0;
-    for (size_t pi = 0; pi < ctx->dct.size(); ++pi) {
-      const DctDev& D = ctx->dct[pi];
-      struct Ax { long long f, p, P, R; int U, V, ld; long long cU, cV; };
-      const Ax axes[3] = {{D.fX, D.pX, D.PX, D.RX, D.h, D.d, D.h, D.ch, D.cd},
-                          {D.fY, D.pY, D.PY, D.RY, D.w, D.d, D.wp, D.cw, D.cd},
-                          {D.fZ, D.pZ, D.PZ, D.RZ, D.w, D.h, D.wp, D.cw, D.ch}};
-      for (const Ax& a : axes) {
-        const long long LS = (long long)a.V * a.ld;
-        const long long UU = (long long)a.U * a.U, VV = (long long)a.V * a.V;
-        const long long xp = face2d_pitch(a.U), ap = face2d_pitch(a.V);
-        xs = std::max(xs, (long long)a.V * std::max(xp, ap));   // whole jobs (the eligibility of the fused form)
-        x1 = xs;
-        bs = std::max(bs, 32LL * ((a.U + 3) & ~3));
-        ts = std::max(ts, 32LL * ((a.V + 3) & ~3));
-        for (int u0 = 0; u0 < a.U; u0 += 32) {
-          const int ub = std::min(32, a.U - u0);
-          for (int n = 0; n < 3; ++n) {
-            // forward: layers n, 5-n -> even / odd parts P[0][n], P[1][n]
-            Face2DJob j{};
-            j.in0 = a.f + n * LS; j.in1 = a.f + (5 - n) * LS;
-            j.out0 = a.P + n * LS; j.out1 = a.P + (3 + n) * LS;
-            j.tabA = a.cV; j.tabB = a.cU + 2 * UU;
-            j.V = a.V; j.U = a.U; j.ld = a.ld; j.u0 = u0; j.ub = ub; j.scale = D.sf; j.part = (int)pi;
-            ctx->fwd2d.push_back(j);
-            // inverse: even / odd parts (partials summed beforehand) -> layers n, 5-n
-            Face2DJob k{};
-            k.in0 = a.R + n * LS; k.in1 = a.R + (3 + n) * LS;
-            k.out0 = a.p + n * LS; k.out1 = a.p + (5 - n) * LS;
-            k.tabA = a.cV + 3 * VV; k.tabB = a.cU + UU;
-            k.V = a.V; k.U = a.U; k.ld = a.ld; k.u0 = u0; k.ub = ub; k.scale = D.si; k.part = (int)pi;
-            ctx->inv2d.push_back(k);
-          }
-        }
-      }
-    }
-    ctx->f2d_smem = Face2DSmem{(int)xs, (int)x1, (int)bs, (int)ts};
-    ctx->f2d_bytes = (size_t)(xs + x1 + bs + 2 * ts) * es0;
-    ctx->fused_faces = !ctx->dct.empty() && !ctx->tune_gemm &&
-                       ctx->f2d_bytes <= (size_t)std::min(ctx->smem_optin, 200 * 1024);
-  }
   if (ctx->adjoint) build_adjoint_jobs(ctx);
   // every GEMM job list runs as one face_gemm_kernel instance: its jobs must
   // agree on the pass direction, the table orientation and the input pair
@@ -919,12 +939,6 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
           ctx->err = "internal: mixed GEMM job list";
           return ARD_ERR_STATE;
         }
-  }
-  // ---- tensor-core face transforms (FP32, two-pass form; ARD_FACE_MMA=0 keeps the CUDA-core passes) ----
-  {
-    const char* env = std::getenv("ARD_FACE_MMA");
-    ctx->mma_faces = ctx->prec == ARD_PREC_F32 && !ctx->fused_faces && !ctx->dct.empty() && !(env && env[0] == '0');
-    if (ctx->mma_faces) build_mma_jobs(ctx, [&](long long n) { return pool.take(n); });
   }
   // ---- air partition groups: two streams in the step graph when the fused
   // face transforms are used and a split leaves each side >= 20 % of the cells ----
@@ -960,14 +974,27 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     }
   }
   if (ctx->fused_faces) {
-    // CTAs of one wave: two per SM (the kernel's bound; the shared memory of
-    // row-split jobs, sized below, is about half that of whole ones)
+    // blocks of one wave: two per SM (the kernel's bound)
     const int slots = ctx->num_sms * 2;
+    // whole jobs that would leave one block per SM are split by output
+    auto presplit = [&](std::vector<Face2DJob>* list, bool inverse) {
+      for (size_t i = 0, n = list->size(); i < n; ++i) {
+        const FaceSmem m = face_smem((*list)[i], 0, inverse);
+        if ((size_t)(m.f + m.a + m.b + m.t) * elem_size(ctx) <= 96 * 1024) continue;
+        (*list)[i].which = 1;
+        list->push_back((*list)[i]);
+        list->back().which = 2;
+      }
+    };
+    presplit(&ctx->fwd2d, false);
+    presplit(&ctx->inv2d, true);
+    presplit(&ctx->adj1_2d, false);
+    presplit(&ctx->adj2_2d, true);
     // each group gets a share of one wave in proportion to its arithmetic
     auto grouped = [&](std::vector<Face2DJob>* list, auto set_range) {
       if (ctx->ngroups == 1) {
-        const bool sp = balance_face_jobs(list, slots);
-        set_range(0, 0, (int)list->size() / 2, sp);
+        balance_face_jobs(list, slots);
+        set_range(0, 0, (int)list->size() / 2);
         return;
       }
       std::vector<Face2DJob> parts[2];
@@ -975,39 +1002,37 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
       for (const Face2DJob& j : *list) {
         const int g = j.part >= ctx->groups[1].part_lo ? 1 : 0;
         parts[g].push_back(j);
-        w[g] += (double)j.V * (j.U + j.V) * j.ub;
+        w[g] += (double)j.V * (j.U + j.V) * j.ub * (j.which == 0 ? 2 : 1);
       }
       list->clear();
       for (int g = 0; g < 2; ++g) {
         const int sg = std::max(1, (int)std::lround(slots * w[g] / std::max(1.0, w[0] + w[1])));
-        const bool sp = balance_face_jobs(&parts[g], sg);
+        balance_face_jobs(&parts[g], sg);
         const int lo = (int)list->size() / 2;
         list->insert(list->end(), parts[g].begin(), parts[g].end());
-        set_range(g, lo, (int)list->size() / 2, sp);
+        set_range(g, lo, (int)list->size() / 2);
       }
     };
-    grouped(&ctx->fwd2d, [&](int g, int lo, int hi, bool sp) {
-      ctx->groups[g].f_lo = lo; ctx->groups[g].f_hi = hi; ctx->groups[g].f_split = sp;
-    });
-    grouped(&ctx->inv2d, [&](int g, int lo, int hi, bool sp) {
-      ctx->groups[g].i_lo = lo; ctx->groups[g].i_hi = hi; ctx->groups[g].i_split = sp;
-    });
-    ctx->adj1_split = balance_face_jobs(&ctx->adj1_2d, slots);
-    ctx->adj2_split = balance_face_jobs(&ctx->adj2_2d, slots);
-    // shared memory of the balanced jobs: a CTA stages its rows of the layers
-    // (all V, or half of a split job) and all of T
-    const size_t es0 = elem_size(ctx);
-    long long xs = 0, bs = 0, ts = 0;
-    for (const std::vector<Face2DJob>* L : {&ctx->fwd2d, &ctx->inv2d, &ctx->adj1_2d, &ctx->adj2_2d})
-      for (const Face2DJob& j : *L) {
-        if (j.V == 0) continue;
-        const long long rows = j.split ? (j.V + 1) / 2 : j.V;
-        xs = std::max(xs, rows * std::max(face2d_pitch(j.U), face2d_pitch(j.V)));
-        bs = std::max(bs, 32LL * ((j.U + 3) & ~3));
-        ts = std::max(ts, 32LL * ((j.V + 3) & ~3));
+    grouped(&ctx->fwd2d, [&](int g, int lo, int hi) { ctx->groups[g].f_lo = lo; ctx->groups[g].f_hi = hi; });
+    grouped(&ctx->inv2d, [&](int g, int lo, int hi) { ctx->groups[g].i_lo = lo; ctx->groups[g].i_hi = hi; });
+    balance_face_jobs(&ctx->adj1_2d, slots);
+    balance_face_jobs(&ctx->adj2_2d, slots);
+    FaceSmem sm{0, 0, 0, 0};
+    auto widen = [&](const std::vector<Face2DJob>& list, bool inverse) {
+      for (size_t i = 0; i < list.size(); ++i) {
+        if (list[i].V == 0) continue;
+        const FaceSmem m = face_smem(list[i], (int)(i & 1), inverse);
+        sm = FaceSmem{std::max(sm.f, m.f), std::max(sm.a, m.a), std::max(sm.b, m.b), std::max(sm.t, m.t)};
       }
-    ctx->f2d_smem = Face2DSmem{(int)xs, (int)xs, (int)bs, (int)ts};
-    ctx->f2d_bytes = (size_t)(2 * xs + bs + 2 * ts) * es0;
+    };
+    widen(ctx->fwd2d, false);
+    widen(ctx->inv2d, true);
+    widen(ctx->adj1_2d, false);
+    widen(ctx->adj2_2d, true);
+    auto up4 = [](int v) { return (v + 3) & ~3; };
+    ctx->f2d_smem = FaceSmem{up4(sm.f), up4(sm.a), up4(sm.b), up4(sm.t)};
+    ctx->f2d_bytes = (size_t)(ctx->f2d_smem.f + ctx->f2d_smem.a + ctx->f2d_smem.b + ctx->f2d_smem.t) * elem_size(ctx);
+    if (ctx->f2d_bytes > (size_t)ctx->smem_optin) { ctx->err = "internal: face jobs exceed shared memory"; return ARD_ERR_STATE; }
   }
 
   // ---- device allocation ----
@@ -1080,6 +1105,13 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     const int blocks = (int)std::min<long long>((nn + 255) / 256, 4096);
     if (ctx->prec == ARD_PREC_F64) cos_table_kernel<double><<<blocks, 256, 0, ctx->stream>>>((double*)ctx->d_buf, kv.second, kv.first);
     else cos_table_kernel<float><<<blocks, 256, 0, ctx->stream>>>((float*)ctx->d_buf, kv.second, kv.first);
+    ARD_CUDA(cudaGetLastError());
+  }
+  for (auto& kv : ctx->face_tables) {  // parity-split tables of the fused face transforms
+    const int blocks = (int)std::min<long long>((face_table_elems(kv.first) + 255) / 256, 4096);
+    const long long cos = cos_off[kv.first];
+    if (ctx->prec == ARD_PREC_F64) face_table_kernel<double><<<blocks, 256, 0, ctx->stream>>>((double*)ctx->d_buf, kv.second, cos, kv.first);
+    else face_table_kernel<float><<<blocks, 256, 0, ctx->stream>>>((float*)ctx->d_buf, kv.second, cos, kv.first);
     ARD_CUDA(cudaGetLastError());
   }
   for (auto& kv : ctx->mma_tables) {   // split TF32 tables of the tensor-core face passes (FP32 contexts)
