@@ -105,10 +105,10 @@ int launch_adjoint_step(Ctx* ctx, int t, int tstep, cudaStream_t s, cudaStream_t
     ARD_CUDA(cudaStreamWaitEvent(s2, ctx->ev_fork, 0));
   }
   if (!ctx->pml_blocks.empty()) {
-    PmlAdjArgs<T> pa{buf, ctx->d_pml, ctx->d_pml_blocks, (int)ctx->pml_blocks.size(), lin, ly, lout, (t + 1) & 1,
+    PmlAdjArgs<T> pa{buf, ctx->d_pml, ctx->d_pml_ablocks, (int)ctx->pml_ablocks.size(), lin, ly, lout, (t + 1) & 1,
                      (T)ctx->dt, (T)ctx->dh, (T)ctx->c0, (const T*)hv.p, (const T*)hv.phn, hv.hlen, ctx->d_tb,
                      tstep, hv.gz, ctx->d_pml_amaps, hv.hmaps, ctx->d_err};
-    ARD_CUDA(launch_dep(pml_adjoint_kernel<T>, grid_for((long long)ctx->pml_blocks.size(), 1, ctx->num_sms * 8), 256,
+    ARD_CUDA(launch_dep(pml_adjoint_kernel<T>, grid_for((long long)ctx->pml_ablocks.size(), 1, ctx->num_sms * 8), 256,
                         0, fork ? s2 : s, pa));
     ARD_CUDA(cudaGetLastError());
   }
@@ -336,9 +336,9 @@ int adjoint_impl(Ctx* ctx, long long T_steps, const float* target, int checkpoin
   const int nrec = ctx->n_rec_total, nsrc = ctx->n_src_total;
   ARD_CUDA(cudaMalloc(&ab.resid, std::max<size_t>(1, (size_t)T_steps * nrec * es)));
   ARD_CUDA(cudaMalloc(&ab.gsrc, std::max<size_t>(1, (size_t)T_steps * nsrc * sizeof(double))));
-  ARD_CUDA(cudaMalloc(&ab.gz, std::max<size_t>(1, ctx->pml_blocks.size() * kMaxPmlLayers * sizeof(double))));
+  ARD_CUDA(cudaMalloc(&ab.gz, std::max<size_t>(1, ctx->pml_ablocks.size() * kMaxPmlLayers * sizeof(double))));
   ARD_CUDA(cudaMemsetAsync(ab.gsrc, 0, (size_t)T_steps * nsrc * sizeof(double), s));
-  ARD_CUDA(cudaMemsetAsync(ab.gz, 0, ctx->pml_blocks.size() * kMaxPmlLayers * sizeof(double), s));
+  ARD_CUDA(cudaMemsetAsync(ab.gz, 0, ctx->pml_ablocks.size() * kMaxPmlLayers * sizeof(double), s));
 
   T* buf = reinterpret_cast<T*>(ctx->d_buf);
   T* state = buf + ctx->state_begin;
@@ -472,12 +472,12 @@ int adjoint_impl(Ctx* ctx, long long T_steps, const float* target, int checkpoin
     for (size_t si = 0; si < ctx->scenes.size(); ++si)
       for (int f = 0; f < 6; ++f) grad_scale[si * 6 + f] = 0.f;
     if (need_hist) {
-      std::vector<double> gz(ctx->pml_blocks.size() * kMaxPmlLayers);
+      std::vector<double> gz(ctx->pml_ablocks.size() * kMaxPmlLayers);
       ARD_CUDA(cudaMemcpy(gz.data(), ab.gz, gz.size() * sizeof(double), cudaMemcpyDeviceToHost));
       std::vector<std::vector<double>> per_slab(ctx->pml.size());
       for (size_t k = 0; k < ctx->pml.size(); ++k) per_slab[k].assign(ctx->pml[k].L, 0.0);
-      for (size_t b = 0; b < ctx->pml_blocks.size(); ++b) {
-        const int slab = ctx->pml_blocks[b].x;
+      for (size_t b = 0; b < ctx->pml_ablocks.size(); ++b) {
+        const int slab = ctx->pml_ablocks[b].x;
         for (int l = 0; l < ctx->pml[slab].L; ++l) per_slab[slab][l] += gz[b * kMaxPmlLayers + l];
       }
       std::vector<double> acc(ctx->scenes.size() * 6, 0.0);

@@ -133,7 +133,7 @@ template <typename T>
 struct PmlAdjArgs {
   T* buf;
   const PmlDev* pml;
-  const int4* blocks;   // {slab, a0, b0}: the forward kernel's 8 x 32 plane tiles
+  const int4* blocks;   // {slab, a0, b0}: 8 x 32 plane tiles
   int nblocks;
   int lx, ly, lo;       // adjoint pressure levels of steps t + 1, t + 2 (read, then cleared) and t (accumulated)
   int fin;              // level of the adjoint phi of step t + 1; step t's goes to fin ^ 1
@@ -151,6 +151,9 @@ struct PmlAdjArgs {
   const CUtensorMap* hmaps;   // per slab: the history of p as a [K+1][L][A][B] tensor (null: no gradient)
   int* err;                   // set to 1 when a bounded wait runs out
 };
+
+// Plane tiles of the adjoint PML kernel.
+constexpr int kPmlTA = 8, kPmlTB = 32;
 
 // The adjoint PML kernel's tile boxes per layer (each 128-byte aligned in the
 // stage): X = adjoint p(t+1) with a halo of 3 (x from b0 - 4), Phi_a with a

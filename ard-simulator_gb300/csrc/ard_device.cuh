@@ -97,6 +97,7 @@ struct PmlDev {
   int Bp;                 // row pitch of the plane: B rounded up to 4 (rows start on 16-byte
                           // boundaries, as the tensor-map tile loads of the PML kernel need)
   int strip0;             // first layer of the forced strip (L-3 or 0)
+  int q;                  // plane tile of the forward update (pml_shape)
   int scene;
   long long p[2];
   long long phn[2], pha[2], phb[2];

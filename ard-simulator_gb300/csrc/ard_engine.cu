@@ -100,6 +100,7 @@ static int configure_kernels(Ctx* ctx) {
   // sizes can be interleaved in one process.
   const int f2d = std::max(ctx->smem_optin, (int)ctx->f2d_bytes);
   if (ctx->prec == ARD_PREC_F64) {
+    ARD_CUDA(cudaFuncSetAttribute(pml_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pml_smem_bytes<double>()));
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     if (ctx->fused_faces) {
@@ -107,6 +108,7 @@ static int configure_kernels(Ctx* ctx) {
       ARD_CUDA(cudaFuncSetAttribute(face_kernel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2d));
     }
   } else {
+    ARD_CUDA(cudaFuncSetAttribute(pml_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pml_smem_bytes<float>()));
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     ARD_CUDA(cudaFuncSetAttribute(modal_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, modal_smem));
     if (ctx->fused_faces) {
@@ -440,10 +442,12 @@ int launch_step(Ctx* ctx, int par, int tstep, cudaStream_t s, cudaStream_t s2, b
 template <typename T>
 int launch_pml(Ctx* ctx, int par, int tstep, cudaStream_t s) {
   if (ctx->pml_blocks.empty()) return ARD_OK;
+  const double dt2 = ctx->dt * ctx->dt;
   PmlArgs<T> pa{reinterpret_cast<T*>(ctx->d_buf), ctx->d_pml, ctx->d_pml_blocks, (int)ctx->pml_blocks.size(), par,
-                (T)ctx->dt, (T)ctx->dh, (T)ctx->c0, (const PmlHist<T>*)ctx->d_phist, ctx->d_t, tstep,
-                ctx->d_pml_maps, ctx->d_err};
-  ARD_CUDA(launch_dep(pml_kernel<T>, grid_for((long long)ctx->pml_blocks.size(), 1, ctx->num_sms * 8), 256, 0, s, pa));
+                (T)ctx->dt, (T)dt2, (T)(ctx->c0 * ctx->c0 * dt2 / (180.0 * ctx->dh * ctx->dh)), (T)(1.0 / (12.0 * ctx->dh)),
+                (const PmlHist<T>*)ctx->d_phist, ctx->d_t, tstep, ctx->d_pml_maps, ctx->d_err};
+  ARD_CUDA(launch_dep(pml_kernel<T>, grid_for((long long)ctx->pml_blocks.size(), 1, ctx->num_sms * pml_blocks_per_sm<T>()),
+                      kPmlThreads, pml_smem_bytes<T>(), s, pa));
   ARD_CUDA(cudaGetLastError());
   return ARD_OK;
 }

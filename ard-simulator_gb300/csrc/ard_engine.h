@@ -65,7 +65,7 @@ struct Ctx {
   std::vector<SceneRec> scenes;
   std::vector<DctDev> dct;
   std::vector<PmlDev> pml;
-  std::vector<int4> pml_blocks;
+  std::vector<int4> pml_blocks, pml_ablocks;   // plane tiles: forward, adjoint (options.adjoint)
   std::vector<IfaceDev> ifs;
   std::vector<unsigned char> masks;
   std::vector<int> cell_iface;              // interface of every face cell
@@ -131,6 +131,7 @@ struct Ctx {
   DctDev* d_dct = nullptr;
   PmlDev* d_pml = nullptr;
   int4* d_pml_blocks = nullptr;
+  int4* d_pml_ablocks = nullptr;
   IfaceDev* d_ifs = nullptr;
   int* d_cell_iface = nullptr;
   PointDev* d_srcpts = nullptr;

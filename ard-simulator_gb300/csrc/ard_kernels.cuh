@@ -684,10 +684,11 @@ template <typename T>
 struct PmlArgs {
   T* buf;
   const PmlDev* pml;
-  const int4* blocks;   // {slab, a0, b0}: 8 x 32 plane tiles
+  const int4* blocks;   // {slab, a0, b0}: plane tiles (pml_shape)
   int nblocks;
   int par;
-  T dt, dh, c0;
+  T dt, dt2;
+  T klap, r12;          // c0^2 dt^2 / (180 dh^2), 1 / (12 dh)
   const PmlHist<T>* hist;   // null without the adjoint
   const long long* tcount;
   int tstep;
@@ -695,47 +696,90 @@ struct PmlArgs {
   int* err;                 // set to 1 when a bounded wait runs out
 };
 
-// Plane tiles of the PML kernel and the boxes the TMA unit loads per layer:
-// p with a halo of 3 along a and of 4 / 4 along b (x starts at b0 - 4, on a
-// 16-byte boundary), phi_a with a halo of 2 along a, phi_b with a halo of 4 /
-// 4 along b; each box 128-byte aligned in the stage.
-constexpr int kPmlTA = 8, kPmlTB = 32;
-template <typename T>
-struct PmlStage {
-  static constexpr int PW = kPmlTB + 8;                                  // p and phi_b box width
-  static constexpr int ps = (kPmlTA + 6) * PW * (int)sizeof(T);
-  static constexpr int psa = (ps + 127) & ~127;
-  static constexpr int fa = (kPmlTA + 4) * kPmlTB * (int)sizeof(T);
-  static constexpr int fb = kPmlTA * PW * (int)sizeof(T);
-  static constexpr int fba = (fb + 127) & ~127;
-  static constexpr int bytes = psa + fa + fba;
-  static constexpr int tx = ps + fa + fb;                                 // bytes the three boxes deliver
+// Plane tile of a slab: a block of kPmlThreads threads, four consecutive b
+// each, 2^q of them along b: 32 x 16, 16 x 32 or 8 x 64 cells (a x b),
+// whichever covers the slab's plane with the fewest tiles.
+constexpr int kPmlThreads = 128;
+constexpr int kPmlStages = 2;   // a third stage measured no faster
+struct PmlShape {
+  int q;        // log2 of the threads along b
+  int TA, TB;   // tile extents
+  int PW;       // row pitch of the p and phi_b boxes
 };
+__host__ __device__ inline PmlShape pml_shape(int q) { return {q, kPmlThreads >> q, 4 << q, (4 << q) + 8}; }
+__host__ __device__ inline int pml_tiles(int q, int A, int B) {
+  const PmlShape s = pml_shape(q);
+  return ((A + s.TA - 1) / s.TA) * ((B + s.TB - 1) / s.TB);
+}
+inline int pml_pick_shape(int A, int B) {
+  int best = 3;
+  for (int q : {2, 4})
+    if (pml_tiles(q, A, B) < pml_tiles(best, A, B)) best = q;
+  return best;
+}
+
+// The boxes that the TMA unit loads per layer: p with a halo of 3 along a and
+// of 4 / 4 along b (x starts at b0 - 4, on a 16-byte boundary), phi_a with a
+// halo of 2 along a, phi_b with a halo of 4 / 4 along b; each box 128-byte
+// aligned in the stage.
+template <typename T>
+struct PmlBoxes {
+  int p, fa, fb;      // bytes
+  int off_fa, off_fb; // offsets in the stage
+  __host__ __device__ explicit PmlBoxes(const PmlShape& s) {
+    p = (s.TA + 6) * s.PW * (int)sizeof(T);
+    fa = (s.TA + 4) * s.TB * (int)sizeof(T);
+    fb = s.TA * s.PW * (int)sizeof(T);
+    off_fa = (p + 127) & ~127;
+    off_fb = off_fa + fa;   // fa is a multiple of 128
+  }
+};
+// bytes of a stage: the largest shape (8 x 64)
+template <typename T>
+__host__ __device__ constexpr int pml_stage_bytes() {
+  return ((14 * 72 * (int)sizeof(T) + 127) & ~127) + 12 * 64 * (int)sizeof(T) + 8 * 72 * (int)sizeof(T) + 128;
+}
+template <typename T>
+constexpr size_t pml_smem_bytes() { return (size_t)kPmlStages * pml_stage_bytes<T>() + 128; }
+template <typename T>
+constexpr int pml_blocks_per_sm() { return sizeof(T) == 4 ? 4 : 2; }
 
 // Grote-Sim PML (pml_partition.cpp:113-200) in slab coordinates: layer l
 // along the normal, (a, b) in the plane; outside the slab every field reads
 // zero (the reference's sentinel cell).  Only the normal damping zeta_n is
 // non-zero in a slab (zeta_a = zeta_b = 0 in the reference's formulas).
-// A block owns an 8 x 32 plane tile and walks the layers.  The in-plane
-// stencils read tiles of p(t-1) (halo 3), phi_a and phi_b (halo 2 along
-// their own axis) that the TMA unit brings into a two-stage ring of shared
-// memory, one layer ahead, across the block's tiles; the tensor maps'
-// zero fill outside the slab is the sentinel.  The normal-axis stencils run
-// from register windows; p(t-2) and the strip force of the next layer are
-// fetched into registers while the current one computes.  Every wait is
-// bounded: one that runs out sets the kernel's error word and the block
-// leaves its loops.
+// A block owns a plane tile (pml_shape) and walks the layers; a thread owns
+// four consecutive b.  The in-plane stencils read tiles of p(t-1) (halo 3),
+// phi_a and phi_b (halo 2 along their own axis) that the TMA unit brings into
+// a ring of shared memory, ahead of the computation and across the block's
+// tiles; the tensor maps' zero fill outside the slab is the sentinel.  The
+// normal-axis stencils run from register windows; p(t-2) and the strip force
+// of the next layer are fetched into registers while the current one computes.
+// The stencils' symmetric taps are summed before they are weighted (19
+// operations for the three axes' Laplacian instead of 21, 11 for the
+// divergence instead of 15).  Large slabs are bound by HBM and by the chain of
+// a layer at 16 warps per SM (the windows take the registers): GB300, 22.3 M
+// cells 249 -> 178 us (4.5 TB/s of 36 bytes per cell), 20.8 M cells in the
+// slabs of 128 scenes 342 -> 205 us, against one cell per thread and 8 x 32
+// tiles; three blocks per SM 207 and 237 us, five spill (263, 300).  FP64 is
+// bound by its arithmetic (0.22 M cells 98 -> 74 us).  Every wait is bounded:
+// one that runs out sets the kernel's error word and the block leaves its
+// loops.
 template <typename T>
-__global__ void __launch_bounds__(256, 4) pml_kernel(PmlArgs<T> a) {
-  grid_dependency_wait();
-  using S = PmlStage<T>;
-  constexpr int TA = kPmlTA, TB = kPmlTB, PW = S::PW;
-  __shared__ __align__(128) unsigned char stage[2][S::bytes];
-  __shared__ uint64_t bar[2];
+__global__ void __launch_bounds__(kPmlThreads, pml_blocks_per_sm<T>()) pml_kernel(PmlArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned char* const stage =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
+  constexpr int kStage = pml_stage_bytes<T>();
+  __shared__ uint64_t bar[kPmlStages];
   __shared__ volatile int s_abort;
-  const T c7[7] = {2, -27, 270, -490, 270, -27, 2};
-  const T c5[5] = {1, -8, 0, 8, -1};
-  const int tb = threadIdx.x & 31, ta = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < kPmlStages; ++k) mbar_init(&bar[k], 1);
+    mbar_init_fence();
+    s_abort = 0;
+  }
+  grid_dependency_wait();
+  __syncthreads();
   T* hp = nullptr;
   T* hfn = nullptr;
   T* hf = nullptr;
@@ -750,145 +794,197 @@ __global__ void __launch_bounds__(256, 4) pml_kernel(PmlArgs<T> a) {
     if (h.f && t >= h.ft0 && t < h.ft1) hf = h.f + (t - h.ft0) * h.flen;
     if (h.fsrc) fsrc = h.fsrc + (t - h.fs0) * h.flen;
   }
-  if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_init_fence();
-    s_abort = 0;
-  }
-  __syncthreads();
-  // thread 0's issue cursor: the block's (tile, layer) sequence, one layer
-  // ahead of the computation (two stages)
-  int ibi = blockIdx.x, il = 0, iL = 0;
-  uint32_t issued = 0;
+  // thread 0's issue cursor over the block's (tile, layer) sequence
+  int ibi = blockIdx.x, il = 0, iL = 0, iq = 0, ist = 0;
   const int lev = a.par ^ 1;   // time level t-1 of p, phi_a, phi_b
   auto issue_next = [&]() {
     if (ibi >= a.nblocks) return;
     const int4 blk = a.blocks[ibi];
-    if (il == 0) iL = a.pml[blk.x].L;
+    if (il == 0) {
+      iL = a.pml[blk.x].L;
+      iq = a.pml[blk.x].q;
+    }
+    const PmlShape S = pml_shape(iq);
+    const PmlBoxes<T> X(S);
     const CUtensorMap* mp = a.maps + 6LL * blk.x;
-    const int sg = (int)(issued & 1);
-    unsigned char* sb = stage[sg];
-    mbar_arrive_expect_tx(&bar[sg], (uint32_t)S::tx);
-    tma_load_3d(sb, mp + lev, blk.z - 4, blk.y - 3, il, &bar[sg]);
-    tma_load_3d(sb + S::psa, mp + 2 + lev, blk.z, blk.y - 2, il, &bar[sg]);
-    tma_load_3d(sb + S::psa + S::fa, mp + 4 + lev, blk.z - 4, blk.y, il, &bar[sg]);
-    ++issued;
+    unsigned char* sb = stage + ist * kStage;
+    uint64_t* br = &bar[ist];
+    mbar_arrive_expect_tx(br, (uint32_t)(X.p + X.fa + X.fb));
+    tma_load_3d(sb, mp + lev, blk.z - 4, blk.y - 3, il, br);
+    tma_load_3d(sb + X.off_fa, mp + 2 + lev, blk.z, blk.y - 2, il, br);
+    tma_load_3d(sb + X.off_fb, mp + 4 + lev, blk.z - 4, blk.y, il, br);
+    ist = ist + 1 == kPmlStages ? 0 : ist + 1;
     if (++il == iL) {
       il = 0;
       ibi += gridDim.x;
     }
   };
-  if (threadIdx.x == 0) {
-    issue_next();
-    issue_next();
-  }
-  uint32_t used = 0;   // layers consumed by the block (uniform)
+  if (threadIdx.x == 0)
+    for (int k = 0; k < kPmlStages; ++k) issue_next();
+  int sg = 0;           // stage and phase of the layer being computed (uniform)
+  uint32_t phase = 0;
   bool stop = false;
   for (int bi = blockIdx.x; bi < a.nblocks && !stop; bi += gridDim.x) {
     const int4 blk = a.blocks[bi];
     const PmlDev& P = a.pml[blk.x];
     const int L = P.L, A = P.A, B = P.B, Bp = P.Bp;
+    const PmlShape S = pml_shape(P.q);
+    const PmlBoxes<T> X(S);
+    const int PW = S.PW, TB = S.TB;
+    const int tb = 4 * ((int)threadIdx.x & ((1 << S.q) - 1)), ta = (int)threadIdx.x >> S.q;
     const int strip0 = P.strip0;       // held in registers: the layer loop stores through the pool pointer
     const long long hoff = P.hoff;
-    const int a0 = blk.y, b0 = blk.z;
-    const int ia = a0 + ta, ib = b0 + tb;
+    const int ia = blk.y + ta, ib = blk.z + tb;
     const bool inside = ia < A && ib < B;
+    const int nb = B - ib;             // cells of the thread's four that lie in the slab
     const long long lstride = (long long)A * Bp;
     const long long col = inside ? (long long)ia * Bp + ib : 0;
-    const T* p = a.buf + P.p[a.par ^ 1];   // p(t-1)
-    T* pn = a.buf + P.p[a.par];            // p(t-2) -> p(t)
-    const T* fn = a.buf + P.phn[a.par ^ 1];
-    T* fn_o = a.buf + P.phn[a.par];
-    T* fa_o = a.buf + P.pha[a.par];
-    T* fb_o = a.buf + P.phb[a.par];
+    const T* p = a.buf + P.p[a.par ^ 1] + col;   // p(t-1)
+    T* pn = a.buf + P.p[a.par] + col;            // p(t-2) -> p(t)
+    const T* fn = a.buf + P.phn[a.par ^ 1] + col;
+    T* fn_o = a.buf + P.phn[a.par] + col;
+    T* fa_o = a.buf + P.pha[a.par] + col;
+    T* fb_o = a.buf + P.phb[a.par] + col;
     const T* zeta = a.buf + P.zeta;
-    const T* force = fsrc ? fsrc + P.foff : a.buf + P.force;
-    T* force_rec = hf ? hf + P.foff : nullptr;
+    const T* force = (fsrc ? fsrc + P.foff : a.buf + P.force) + col;
+    T* force_rec = hf ? hf + P.foff + col : nullptr;
+    auto quad = [&](const T* q, bool ok, T (&v)[4]) {
+      if (ok) {
+        load4(q, v);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = 0;
+      }
+    };
     // register windows along the normal: p(l-3 .. l+3), phi_n(l-2 .. l+2)
-    T pw[7], fw[5];
+    T pw[7][4], fw[5][4];
 #pragma unroll
-    for (int m = 0; m < 7; ++m) {
-      const int ll = m - 3;
-      pw[m] = (inside && ll >= 0 && ll < L) ? p[ll * lstride + col] : (T)0;
-    }
+    for (int m = 0; m < 7; ++m) quad(p + (m - 3) * lstride, inside && m >= 3 && m - 3 < L, pw[m]);
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      const int ll = m - 2;
-      fw[m] = (inside && ll >= 0 && ll < L) ? fn[ll * lstride + col] : (T)0;
-    }
-    const T r180 = (T)1 / ((T)180 * a.dh * a.dh), r12 = (T)1 / ((T)12 * a.dh), rdt = (T)1 / a.dt;
-    T nold = 0, nforce = 0;
+    for (int m = 0; m < 5; ++m) quad(fn + (m - 2) * lstride, inside && m >= 2 && m - 2 < L, fw[m]);
+    T nold[4], nforce[4];
     auto fetch = [&](int l) {
       const int sl = l - strip0;
-      nold = inside ? pn[l * lstride + col] : (T)0;
-      nforce = (inside && sl >= 0 && sl < 3) ? force[sl * lstride + col] : (T)0;
+      quad(pn + l * lstride, inside, nold);
+      quad(force + sl * lstride, inside && sl >= 0 && sl < 3, nforce);
     };
     fetch(0);
     for (int l = 0; l < L; ++l) {
-      const int sg = (int)(used & 1);
-      mbar_wait_bounded(&bar[sg], (used >> 1) & 1, &s_abort);
-      const T* Ps = reinterpret_cast<const T*>(stage[sg]);                    // [TA + 6][PW], b from b0 - 4
-      const T* FA = reinterpret_cast<const T*>(stage[sg] + S::psa);           // [TA + 4][TB], b from b0
-      const T* FB = reinterpret_cast<const T*>(stage[sg] + S::psa + S::fa);   // [TA][PW], b from b0 - 4
-      const T pold = nold, f = nforce;
+      T pold[4], f[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        pold[e] = nold[e];
+        f[e] = nforce[e];
+      }
       if (l + 1 < L) fetch(l + 1);
       if (force_rec && inside) {
         const int sl = l - strip0;
-        if (sl >= 0 && sl < 3) force_rec[sl * lstride + col] = f;
+        if (sl >= 0 && sl < 3) store4(force_rec + sl * lstride, f);
       }
+      const T zn = zeta[l];
+      mbar_wait_bounded(&bar[sg], phase, &s_abort);
       if (inside && !s_abort) {
-        T ln = 0, la = 0, lb = 0;
+        const unsigned char* sb = stage + sg * kStage;
+        const T* Ps = reinterpret_cast<const T*>(sb) + ta * PW + tb + 4;                  // rows ia - 3 .., columns ib ..
+        const T* FA = reinterpret_cast<const T*>(sb + X.off_fa) + ta * TB + tb;           // rows ia - 2 ..
+        const T* FB = reinterpret_cast<const T*>(sb + X.off_fb) + ta * PW + tb + 4;
+        T s1[4], s2[4], s3[4], g1[4], g2[4], ua[4], ub[4], v[4], u[4];
+        // along a: p
+        load4(Ps, v); load4(Ps + 6 * PW, u);
 #pragma unroll
-        for (int m = 0; m < 7; ++m) {
-          ln += c7[m] * pw[m];
-          la += c7[m] * Ps[(ta + m) * PW + tb + 4];
-          lb += c7[m] * Ps[(ta + 3) * PW + tb + 1 + m];
-        }
-        T un = 0, ua = 0, ub = 0, gn = 0, ga = 0, gb = 0;
+        for (int e = 0; e < 4; ++e) s3[e] = (v[e] + u[e]) + (pw[0][e] + pw[6][e]);
+        load4(Ps + PW, v); load4(Ps + 5 * PW, u);
 #pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          un += c5[m] * pw[m + 1];
-          ua += c5[m] * Ps[(ta + 1 + m) * PW + tb + 4];
-          ub += c5[m] * Ps[(ta + 3) * PW + tb + 2 + m];
-          gn += c5[m] * fw[m];
-          ga += c5[m] * FA[(ta + m) * TB + tb];
-          gb += c5[m] * FB[ta * PW + tb + 2 + m];
+        for (int e = 0; e < 4; ++e) { s2[e] = (v[e] + u[e]) + (pw[1][e] + pw[5][e]); ua[e] = v[e] - u[e]; }
+        load4(Ps + 2 * PW, v); load4(Ps + 4 * PW, u);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { s1[e] = (v[e] + u[e]) + (pw[2][e] + pw[4][e]); ua[e] += (T)8 * (u[e] - v[e]); }
+        // along b: p
+        {
+          T w[12];
+          load4(Ps + 3 * PW - 4, v); load4(Ps + 3 * PW + 4, u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { w[e] = v[e]; w[4 + e] = pw[3][e]; w[8 + e] = u[e]; }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s3[e] += w[e + 1] + w[e + 7];
+            s2[e] += w[e + 2] + w[e + 6];
+            s1[e] += w[e + 3] + w[e + 5];
+            ub[e] = (w[e + 2] - w[e + 6]) + (T)8 * (w[e + 5] - w[e + 3]);
+          }
         }
-        ln *= r180; la *= r180; lb *= r180;
-        un *= r12; ua *= r12; ub *= r12;
-        gn *= r12; ga *= r12; gb *= r12;
-        const long long I = l * lstride + col;
-        const T zn = zeta[l];
-        const T pcur = pw[3];
-        const T t3 = a.c0 * a.c0 * (ln + la + lb);
-        const T t4 = -zn * (pcur - pold) * rdt;
-        const T pnew = (T)2 * pcur - pold + a.dt * a.dt * (t3 + t4 + (gn + ga + gb) + f);
-        pn[I] = pnew;
-        const T fnc = fw[2];
-        const T fnew = fnc - a.dt * zn * fnc + a.dt * (-zn) * un;
-        fn_o[I] = fnew;
+        // divergence of phi: taps -2, +2 in g2, +1, -1 in g1
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { g2[e] = fw[0][e] - fw[4][e]; g1[e] = fw[3][e] - fw[1][e]; }
+        load4(FA, v); load4(FA + 4 * TB, u);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g2[e] += v[e] - u[e];
+        load4(FA + TB, v); load4(FA + 3 * TB, u);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g1[e] += u[e] - v[e];
+        T fb0[4], fa0[4];
+        load4(FA + 2 * TB, fa0);
+        {
+          T w[12];
+          load4(FB - 4, v); load4(FB, fb0); load4(FB + 4, u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { w[e] = v[e]; w[4 + e] = fb0[e]; w[8 + e] = u[e]; }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            g2[e] += w[e + 2] - w[e + 6];
+            g1[e] += w[e + 5] - w[e + 3];
+          }
+        }
+        const T dz = a.dt * zn, dzr = dz * a.r12, kdiv = a.dt2 * a.r12;
+        T pnew[4], fnew[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const T pc = pw[3][e];
+          const T lap = (T)270 * s1[e] - (T)27 * s2[e] + (T)2 * s3[e] - (T)1470 * pc;
+          const T div = g2[e] + (T)8 * g1[e];
+          const T un = (pw[1][e] - pw[5][e]) + (T)8 * (pw[4][e] - pw[2][e]);
+          pnew[e] = ((T)2 * pc - pold[e]) + (a.klap * lap - dz * (pc - pold[e]) + kdiv * div + a.dt2 * f[e]);
+          const T fc = fw[2][e];
+          fnew[e] = fc - dz * fc - dzr * un;
+          fa0[e] += dzr * ua[e];
+          fb0[e] += dzr * ub[e];
+        }
+        if (nb < 4) {   // the row pitch's padding columns stay zero
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (e >= nb) pnew[e] = fnew[e] = fa0[e] = fb0[e] = 0;
+        }
+        const long long I = l * lstride;
+        store4(pn + I, pnew);
+        store4(fn_o + I, fnew);
+        store4(fa_o + I, fa0);
+        store4(fb_o + I, fb0);
         if (hp) {
-          hp[hoff + I] = pnew;
-          hfn[hoff + I] = fnew;
+          store4(hp + hoff + col + I, pnew);
+          store4(hfn + hoff + col + I, fnew);
         }
-        fa_o[I] = FA[(ta + 2) * TB + tb] + a.dt * zn * ua;
-        fb_o[I] = FB[ta * PW + tb + 4] + a.dt * zn * ub;
       }
       // slide the windows one layer
 #pragma unroll
-      for (int m = 0; m < 6; ++m) pw[m] = pw[m + 1];
-      pw[6] = (inside && l + 4 < L) ? p[(l + 4) * lstride + col] : (T)0;
+      for (int m = 0; m < 6; ++m)
 #pragma unroll
-      for (int m = 0; m < 4; ++m) fw[m] = fw[m + 1];
-      fw[4] = (inside && l + 3 < L) ? fn[(l + 3) * lstride + col] : (T)0;
+        for (int e = 0; e < 4; ++e) pw[m][e] = pw[m + 1][e];
+      quad(p + (l + 4) * lstride, inside && l + 4 < L, pw[6]);
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) fw[m][e] = fw[m + 1][e];
+      quad(fn + (l + 3) * lstride, inside && l + 3 < L, fw[4]);
       __syncthreads();   // every thread is done with stage sg
       if (s_abort) {
         stop = true;
         break;
       }
       if (threadIdx.x == 0) issue_next();
-      ++used;
+      if (++sg == kPmlStages) {
+        sg = 0;
+        phase ^= 1;
+      }
     }
   }
   if (s_abort) {

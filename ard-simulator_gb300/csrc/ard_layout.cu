@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "ard_adjoint_kernels.cuh"
 #include "ard_device.cuh"
 #include "ard_engine.h"
 #include "ard_gb300.h"
@@ -624,7 +625,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     ctx->scratch = pool.take(3 * maxN);
   }
 
-  // ---- PML arrays and 8 x 32 plane tiles ----
+  // ---- PML arrays and plane tiles ----
   for (size_t k = 0; k < ctx->pml.size(); ++k) {
     PmlDev& P = ctx->pml[k];
     if (P.L > kMaxPmlLayers) {
@@ -633,8 +634,12 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     }
     P.zeta = pool.take(P.L);
     ctx->n_pml_cells += (long long)P.L * P.A * P.B;
-    for (int a0 = 0; a0 < P.A; a0 += 8)
-      for (int b0 = 0; b0 < P.B; b0 += 32) ctx->pml_blocks.push_back(make_int4((int)k, a0, b0, 0));
+    P.q = pml_pick_shape(P.A, P.B);
+    const PmlShape S = pml_shape(P.q);
+    for (int a0 = 0; a0 < P.A; a0 += S.TA)
+      for (int b0 = 0; b0 < P.B; b0 += S.TB) ctx->pml_blocks.push_back(make_int4((int)k, a0, b0, 0));
+    for (int a0 = 0; ctx->adjoint && a0 < P.A; a0 += kPmlTA)
+      for (int b0 = 0; b0 < P.B; b0 += kPmlTB) ctx->pml_ablocks.push_back(make_int4((int)k, a0, b0, 0));
   }
 
   // ---- interfaces + owner masks ----
@@ -1084,6 +1089,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
   ARD_CUDA(cudaMemset(ctx->d_err, 0, sizeof(int)));
   if (int rc = build_tensor_maps(ctx)) return rc;
   if (ctx->adjoint) {
+    if ((rc = up(&ctx->d_pml_ablocks, ctx->pml_ablocks))) return rc;
     if ((rc = up(&ctx->d_adj1_2d, ctx->adj1_2d))) return rc;
     if ((rc = up(&ctx->d_adj2_2d, ctx->adj2_2d))) return rc;
     for (int k = 0; k < 4; ++k)
@@ -1150,7 +1156,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
 void free_ctx_device(Ctx* ctx) {
   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
   free_cubes(ctx);
-  void* ptrs[] = {ctx->d_buf_base, ctx->d_mask, ctx->d_dct, ctx->d_pml, ctx->d_pml_blocks, ctx->d_ifs, ctx->d_srcpts,
+  void* ptrs[] = {ctx->d_buf_base, ctx->d_mask, ctx->d_dct, ctx->d_pml, ctx->d_pml_blocks, ctx->d_pml_ablocks, ctx->d_ifs, ctx->d_srcpts,
                   ctx->d_recpts, ctx->d_tiles, ctx->d_fwd1, ctx->d_fwd2, ctx->d_inv1, ctx->d_inv2, ctx->d_fwd2d,
                   ctx->d_inv2d, ctx->d_series,
                   ctx->d_hist, ctx->d_t, ctx->d_adj1_2d, ctx->d_adj2_2d, ctx->d_adjg[0], ctx->d_adjg[1],
@@ -1226,7 +1232,7 @@ static int encode_slab_map(Ctx* ctx, CUtensorMap* map, const PmlDev& P, const vo
 //    of each array, the transformed Y layers as [6][d][wp] in boxes of one
 //    plane's 32 kx of all six;
 //  - the PML kernels' tile loads, with the box of the tile each one feeds
-//    (PmlStage, PmlAdjStage): per slab p (halo 3, x from b0 - 4), phi_a (halo
+//    (PmlBoxes, PmlAdjStage): per slab p (halo 3, x from b0 - 4), phi_a (halo
 //    2 along a) and phi_b (halo 2 along b, x from b0 - 4) of both time levels;
 //    with the adjoint also its three levels of p and two of each phi.
 int build_tensor_maps(Ctx* ctx) {
@@ -1265,8 +1271,11 @@ int build_tensor_maps(Ctx* ctx) {
   for (size_t k = 0; k < ctx->pml.size(); ++k) {
     const PmlDev& P = ctx->pml[k];
     const long long offs[6] = {P.p[0], P.p[1], P.pha[0], P.pha[1], P.phb[0], P.phb[1]};
+    const PmlShape S = pml_shape(P.q);
+    const cuuint32_t fb[3] = {(cuuint32_t)S.PW, (cuuint32_t)S.TB, (cuuint32_t)S.PW},
+                     fa[3] = {(cuuint32_t)S.TA + 6, (cuuint32_t)S.TA + 4, (cuuint32_t)S.TA};
     for (int q = 0; q < 6; ++q)
-      if (int rc = encode_slab_map(ctx, &maps[n_modal + 6 * k + q], P, base + offs[q] * es, bb[q / 2], ba[q / 2]))
+      if (int rc = encode_slab_map(ctx, &maps[n_modal + 6 * k + q], P, base + offs[q] * es, fb[q / 2], fa[q / 2]))
         return rc;
     if (ctx->adjoint) {
       const long long aoffs[7] = {P.ap[0], P.ap[1], P.ap[2], P.apha[0], P.apha[1], P.aphb[0], P.aphb[1]};
