@@ -165,6 +165,8 @@ struct Ctx {
   cudaStream_t stream = nullptr, stream2 = nullptr, stream3 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  cudaGraphExec_t step_exec[2] = {nullptr, nullptr};   // one step of parity 0, 1
+  int direct_steps = 0;           // steps launched kernel by kernel so far
   long long t_host = 0;
 };
 
@@ -183,6 +185,7 @@ int launch_steps_direct(Ctx* ctx, int n, cudaStream_t s);
 template <typename T>
 int launch_pml(Ctx* ctx, int par, int tstep, cudaStream_t s);
 int ensure_graph(Ctx* ctx);
+void free_graphs(Ctx* ctx);
 int check_guards(Ctx* ctx);
 int check_device_error(Ctx* ctx);
 template <typename T>

@@ -1154,7 +1154,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
 }
 
 void free_ctx_device(Ctx* ctx) {
-  if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
+  free_graphs(ctx);
   free_cubes(ctx);
   void* ptrs[] = {ctx->d_buf_base, ctx->d_mask, ctx->d_dct, ctx->d_pml, ctx->d_pml_blocks, ctx->d_pml_ablocks, ctx->d_ifs, ctx->d_srcpts,
                   ctx->d_recpts, ctx->d_tiles, ctx->d_fwd1, ctx->d_fwd2, ctx->d_inv1, ctx->d_inv2, ctx->d_fwd2d,
@@ -1172,7 +1172,6 @@ void free_ctx_device(Ctx* ctx) {
   if (ctx->stream3) cudaStreamDestroy(ctx->stream3);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->stream2) cudaStreamDestroy(ctx->stream2);
-  ctx->graph_exec = nullptr;
   ctx->d_buf = nullptr;
   ctx->d_buf_base = nullptr;
 }

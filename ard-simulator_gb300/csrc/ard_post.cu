@@ -399,10 +399,7 @@ extern "C" int ard_record_neighbourhoods(ard_ctx* c, int32_t enable) {
   ARD_CUDA(cudaSetDevice(ctx->device));
   ARD_CUDA(cudaStreamSynchronize(ctx->stream));
   ARD_CUDA(cudaStreamSynchronize(ctx->stream2));
-  if (ctx->graph_exec) {   // the step graph is captured again with (or without) the cube launches
-    cudaGraphExecDestroy(ctx->graph_exec);
-    ctx->graph_exec = nullptr;
-  }
+  free_graphs(ctx);   // the step graphs are captured again with (or without) the cube launches
   free_cubes(ctx);
   if (!enable) return ARD_OK;
   if (ctx->recpts.empty()) { ctx->err = "ard_record_neighbourhoods: the context has no recorders"; return ARD_ERR_STATE; }
