@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
   T* const Bs = As + sm.a;
   T* const Ts = Bs + sm.b;
   const int tid = threadIdx.x;
-  grid_dependency_wait();
+  bool waited = false;   // jobs and tables are constants: loaded while the predecessor drains
   for (int it = blockIdx.x; it < entries; it += gridDim.x) {
     const Face2DJob J = jobs[it];
     const FaceShape s = face_shape(J, it & 1, INV);
@@ -195,6 +195,10 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
     for (int i = tid; i < units * (hv4 - hv) * ncp; i += kFaceThreads) {   // rows past the half length read as zero
       const int u = i / ((hv4 - hv) * ncp);
       Ts[(u * hv4 + hv) * ncp + i - u * (hv4 - hv) * ncp] = (T)0;
+    }
+    if (!waited) {
+      grid_dependency_wait();
+      waited = true;
     }
     // ---- the layers, combined and folded (or sorted by parity) ----
     const T* X[2] = {buf + J.in0, buf + J.in1};
@@ -286,6 +290,7 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
     if (wide) face_product<T, 4>(units, hv, hu4, nq, fp, ncp, f_of, b_of, to_t);
     else      face_product<T, 2>(units, hv, hu4, nq, fp, ncp, f_of, b_of, to_t);
     __syncthreads();
+    if (it + (int)gridDim.x >= entries) grid_launch_dependents();
     // ---- O = A T ----
     const T scale = (T)J.scale;
     auto a_of = [&](int u) { return As + (u / npu % 2) * hv * ap; };
@@ -325,6 +330,7 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
       }
     }
   }
+  if (!waited) grid_dependency_wait();   // no job: still not done before the predecessor
 }
 
 // Launch over a list of 2 n entries, at most max_ctas blocks.

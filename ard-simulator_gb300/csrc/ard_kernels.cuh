@@ -99,9 +99,22 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // Programmatic dependent launch: a step kernel launched with programmatic
 // stream serialization may start while its predecessor in the stream is
 // finishing; griddepcontrol.wait returns once the predecessor has completed
-// and its writes are visible (at once for an ordinary launch).  Every step
-// kernel waits before its first global access.
+// and its writes are visible (at once for an ordinary launch).  Every block of
+// every step kernel waits, before its first access to what a step kernel
+// writes (constants - descriptors, job lists, tables - may be read before):
+// since each kernel waits for its predecessor and that one for its own, all
+// earlier writes are visible after it.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// Lets the successor's blocks be scheduled once every block of this grid has
+// got here (or ended).  Called where a block has little left to do: the
+// successor's launch and constant loads then lie under this grid's last part
+// (2-3 % of a step of a single room).  Earlier, its waiting blocks would hold
+// the slots of the streams beside it (at kernel entry: L-shaped room 75 -> 96
+// us per step).
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
 
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
@@ -559,16 +572,16 @@ struct PostModalArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) post_modal_kernel(PostModalArgs<T> a) {
-  grid_dependency_wait();
   if ((int)blockIdx.x < a.rec_blocks) {
     const int lane = threadIdx.x & 31;
     const int rl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (rl >= a.nrec) return;
-    const int r = a.rec_first + rl;
+    const int r = a.rec_first + min(rl, a.nrec - 1);
     const PointDev q = a.recs[r];
     const DctDev& D = a.dct[q.part];
     const int local_r = r - D.rec0;
     const int ntiles = D.ntiles;
+    grid_dependency_wait();
+    if (rl >= a.nrec) return;
     T s = 0;
     for (int i = lane; i < ntiles; i += 32) s += a.buf[D.recpart + (long long)i * D.nrec + local_r];
     s = warp_sum(s);
@@ -584,6 +597,7 @@ __global__ void __launch_bounds__(256) post_modal_kernel(PostModalArgs<T> a) {
   if (cached)
     for (int i = threadIdx.x; i < a.njobs; i += blockDim.x) sfirst[i] = a.jobs[i].first;
   __syncthreads();
+  grid_dependency_wait();   // the jobs are constants
   // chunks of kSumChunk elements: a job's elements start on a chunk boundary
   // of the index space, so a chunk lies in one job; a thread sums 8 elements
   // (256 apart) over the job's slabs, slab by slab in order

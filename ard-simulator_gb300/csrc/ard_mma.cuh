@@ -178,7 +178,6 @@ struct MmaSlot {
 };
 
 static __global__ void __launch_bounds__(kMmaThreads, 1) face_mma_kernel(MmaArgs a) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   extern __shared__ __align__(1024) unsigned char mma_smem_raw[];
   // 1024-byte aligned stage area (the swizzle pattern is anchored at 1024-byte boundaries)
   unsigned char* sm = reinterpret_cast<unsigned char*>(
@@ -215,6 +214,7 @@ static __global__ void __launch_bounds__(kMmaThreads, 1) face_mma_kernel(MmaArgs
   const bool cached = a.njobs <= kMaxCachedJobs;
   if (cached)
     for (int i = tid; i < a.njobs; i += kMmaThreads) sfirst[i] = a.jobs[i].first;
+  grid_dependency_wait();   // the data rows are read below; jobs and tables are constants
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -149,10 +149,7 @@ __global__ void __launch_bounds__(kModalThreads, modal_blocks_per_sm<T>()) modal
     mbar_init_fence();
     s_abort = 0;
   }
-  grid_dependency_wait();
-  __syncthreads();
   T* __restrict__ buf = a.buf;
-  const long long t = ADJ ? (*a.tcount - a.tstep) : (*a.tcount + a.tstep);
 
   // thread 0's issue cursor over the block's (tile, plane) sequence
   int itile = blockIdx.x, ipl = 0, ist = 0;
@@ -179,8 +176,19 @@ __global__ void __launch_bounds__(kModalThreads, modal_blocks_per_sm<T>()) modal
     ist = ist + 1 == kModalStages ? 0 : ist + 1;
     ++ipl;
   };
-  if (tid == 0)
-    for (int s = 0; s < kModalStages; ++s) issue_next();
+  // Nothing that an earlier kernel writes is read before this point of the
+  // block's first tile: its descriptors and basis rows are loaded while the
+  // predecessor drains.
+  long long t = 0;
+  bool waited = false;
+  auto wait_predecessor = [&]() {
+    grid_dependency_wait();
+    __syncthreads();   // the barriers are initialised
+    t = ADJ ? (*a.tcount - a.tstep) : (*a.tcount + a.tstep);
+    if (tid == 0)
+      for (int s = 0; s < kModalStages; ++s) issue_next();
+    waited = true;
+  };
 
   const int li = lane & 7, yrow = lane >> 3;
   const int rs = warp * 8 + yrow;     // the thread's ky rows in the tile: rs and rs + 4 (same parity)
@@ -208,6 +216,23 @@ __global__ void __launch_bounds__(kModalThreads, modal_blocks_per_sm<T>()) modal
     const T* Cw = buf + D.cw;
     const T* Ch = buf + D.ch;
     const T* Cd = buf + D.cd;
+    // basis rows: cx[n] as (even, odd) kx pairs, cy[n]; the REDFT01 halving of
+    // the k = 0 rows sits in the contraction (forward) or the expansion (adjoint)
+    bool act[4];
+    Pair<T> cx[3][2];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      act[e] = kx0 + e < w;
+      const T* c = Cw + (long long)min(kx0 + e, w - 1) * w;
+#pragma unroll
+      for (int n = 0; n < 3; ++n) (e & 1 ? cx[n][e >> 1].y : cx[n][e >> 1].x) = c[n];
+    }
+    T cy[R][3];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int n = 0; n < 3; ++n) cy[r][n] = rowok[r] ? Ch[(long long)(ky + 4 * r) * h + n] : (T)0;
+    if (!waited) wait_predecessor();
     const T* zsrc = Cd + min(lane, 2);   // per plane: lanes 0-2 the basis row Cd[kz][0..2], lanes 8.. / 16.. the points'
     if (ninj + nout > 0) {
       // injected points (sources; adjoint: recorders) and read-out points
@@ -248,24 +273,11 @@ __global__ void __launch_bounds__(kModalThreads, modal_blocks_per_sm<T>()) modal
       __syncthreads();
     }
 
-    // basis rows: cx[n] as (even, odd) kx pairs, cy[n]; the REDFT01 halving of
-    // the k = 0 rows sits in the contraction (forward) or the expansion (adjoint)
-    bool act[4];
-    Pair<T> cx[3][2];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      act[e] = kx0 + e < w;
-      const T* c = Cw + (long long)min(kx0 + e, w - 1) * w;
-#pragma unroll
-      for (int n = 0; n < 3; ++n) (e & 1 ? cx[n][e >> 1].y : cx[n][e >> 1].x) = c[n];
-    }
-    T cy[R][3];
     Pair<T> pz[R][3][2], rz[R][3][2];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int n = 0; n < 3; ++n) {
-        cy[r][n] = rowok[r] ? Ch[(long long)(ky + 4 * r) * h + n] : (T)0;
         pz[r][n][0] = pz[r][n][1] = rz[r][n][0] = rz[r][n][1] = {0, 0};
         if (colok && rowok[r]) load4(buf + D.PZ + (zpar * 3 + n) * planeZ + (long long)(ky + 4 * r) * wp + kx0, pz[r][n]);
       }
@@ -493,6 +505,7 @@ __global__ void __launch_bounds__(kModalThreads, modal_blocks_per_sm<T>()) modal
       }
     }
     if (stop) break;
+    if (tile_id + (int)gridDim.x >= a.ntiles) grid_launch_dependents();
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (colok && rowok[r]) {
@@ -516,6 +529,7 @@ __global__ void __launch_bounds__(kModalThreads, modal_blocks_per_sm<T>()) modal
     }
     if (ninj + nout > 0) __syncthreads();   // the points' weights and sums are read before the next tile writes its own
   }
+  if (!waited) grid_dependency_wait();   // no tile: still not done before the predecessor
   if (s_abort) {
     // a wait ran out: report it, and give loads still in flight time to land
     // (bounded) before the block's shared memory is released
