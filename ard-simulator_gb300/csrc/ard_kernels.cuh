@@ -769,14 +769,13 @@ constexpr int pml_blocks_per_sm() { return sizeof(T) == 4 ? 4 : 2; }
 // tiles; the tensor maps' zero fill outside the slab is the sentinel.  The
 // normal-axis stencils run from register windows; p(t-2) and the strip force
 // of the next layer are fetched into registers while the current one computes.
-// The stencils' symmetric taps are summed before they are weighted (19
-// operations for the three axes' Laplacian instead of 21, 11 for the
-// divergence instead of 15).  Large slabs are bound by HBM and by the chain of
+// In FP32 the Laplacian sums taps minus the centre before it weights them
+// (rounding, for smooth fields, a fifth of the tap-by-tap chain's).  Large slabs are bound by HBM and by the chain of
 // a layer at 16 warps per SM (the windows take the registers): GB300, 22.3 M
-// cells 249 -> 178 us (4.5 TB/s of 36 bytes per cell), 20.8 M cells in the
-// slabs of 128 scenes 342 -> 205 us, against one cell per thread and 8 x 32
-// tiles; three blocks per SM 207 and 237 us, five spill (263, 300).  FP64 is
-// bound by its arithmetic (0.22 M cells 98 -> 74 us).  Every wait is bounded:
+// cells 249 -> 185 us (4.3 TB/s of 36 bytes per cell), 20.8 M cells in the
+// slabs of 128 scenes 342 -> 213 us, against one cell per thread and 8 x 32
+// tiles; three blocks per SM were 16 % slower, five spill (half as fast).  FP64 is
+// bound by its arithmetic (0.22 M cells 98 -> 80 us).  Every wait is bounded:
 // one that runs out sets the kernel's error word and the block leaves its
 // loops.
 template <typename T>
@@ -902,30 +901,57 @@ __global__ void __launch_bounds__(kPmlThreads, pml_blocks_per_sm<T>()) pml_kerne
         const T* Ps = reinterpret_cast<const T*>(sb) + ta * PW + tb + 4;                  // rows ia - 3 .., columns ib ..
         const T* FA = reinterpret_cast<const T*>(sb + X.off_fa) + ta * TB + tb;           // rows ia - 2 ..
         const T* FB = reinterpret_cast<const T*>(sb + X.off_fb) + ta * PW + tb + 4;
-        T s1[4], s2[4], s3[4], g1[4], g2[4], ua[4], ub[4], v[4], u[4];
-        // along a: p
-        load4(Ps, v); load4(Ps + 6 * PW, u);
+        T lap[4], g1[4], g2[4], ua[4], ub[4], v[4], u[4], w[12];   // w: p along b from ib - 4
+        load4(Ps + 3 * PW - 4, v); load4(Ps + 3 * PW + 4, u);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s3[e] = (v[e] + u[e]) + (pw[0][e] + pw[6][e]);
-        load4(Ps + PW, v); load4(Ps + 5 * PW, u);
+        for (int e = 0; e < 4; ++e) { w[e] = v[e]; w[4 + e] = pw[3][e]; w[8 + e] = u[e]; }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { s2[e] = (v[e] + u[e]) + (pw[1][e] + pw[5][e]); ua[e] = v[e] - u[e]; }
-        load4(Ps + 2 * PW, v); load4(Ps + 4 * PW, u);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { s1[e] = (v[e] + u[e]) + (pw[2][e] + pw[4][e]); ua[e] += (T)8 * (u[e] - v[e]); }
-        // along b: p
-        {
-          T w[12];
-          load4(Ps + 3 * PW - 4, v); load4(Ps + 3 * PW + 4, u);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) { w[e] = v[e]; w[4 + e] = pw[3][e]; w[8 + e] = u[e]; }
+        for (int e = 0; e < 4; ++e) ub[e] = (w[e + 2] - w[e + 6]) + (T)8 * (w[e + 5] - w[e + 3]);
+        if constexpr (sizeof(T) == 4) {
+          // 2 t3 - 27 t2 + 270 t1, t_m the axes' sums of p(+m) + p(-m) - 2 p:
+          // taps minus the centre cancel before they are weighted (t1 by
+          // differences, which are exact for neighbours within a factor of two)
+          T t1[4], t2[4], t3[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            s3[e] += w[e + 1] + w[e + 7];
-            s2[e] += w[e + 2] + w[e + 6];
-            s1[e] += w[e + 3] + w[e + 5];
-            ub[e] = (w[e + 2] - w[e + 6]) + (T)8 * (w[e + 5] - w[e + 3]);
+            const T pc = pw[3][e], m2 = (T)-2 * pc;
+            t1[e] = ((pw[2][e] - pc) + (pw[4][e] - pc)) + ((w[e + 3] - pc) + (w[e + 5] - pc));
+            t2[e] = ((pw[1][e] + pw[5][e]) + m2) + ((w[e + 2] + w[e + 6]) + m2);
+            t3[e] = ((pw[0][e] + pw[6][e]) + m2) + ((w[e + 1] + w[e + 7]) + m2);
           }
+          load4(Ps, v); load4(Ps + 6 * PW, u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) t3[e] += (v[e] + u[e]) - (T)2 * pw[3][e];
+          load4(Ps + PW, v); load4(Ps + 5 * PW, u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { t2[e] += (v[e] + u[e]) - (T)2 * pw[3][e]; ua[e] = v[e] - u[e]; }
+          load4(Ps + 2 * PW, v); load4(Ps + 4 * PW, u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            t1[e] += (v[e] - pw[3][e]) + (u[e] - pw[3][e]);
+            ua[e] += (T)8 * (u[e] - v[e]);
+            lap[e] = (T)270 * t1[e] - (T)27 * t2[e] + (T)2 * t3[e];
+          }
+        } else {
+          // FP64 is bound by its operations: three weighted chains
+          const T c7[7] = {2, -27, 270, -490, 270, -27, 2};
+          T la[4] = {0, 0, 0, 0}, lb[4] = {0, 0, 0, 0}, ln[4] = {0, 0, 0, 0};
+#pragma unroll
+          for (int m = 0; m < 7; ++m) {
+            load4(Ps + m * PW, v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              la[e] += c7[m] * v[e];
+              lb[e] += c7[m] * w[e + 1 + m];
+              ln[e] += c7[m] * pw[m][e];
+              if (m == 1) ua[e] = v[e];
+              if (m == 2) ua[e] -= (T)8 * v[e];
+              if (m == 4) ua[e] += (T)8 * v[e];
+              if (m == 5) ua[e] -= v[e];
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) lap[e] = ln[e] + la[e] + lb[e];
         }
         // divergence of phi: taps -2, +2 in g2, +1, -1 in g1
 #pragma unroll
@@ -939,7 +965,6 @@ __global__ void __launch_bounds__(kPmlThreads, pml_blocks_per_sm<T>()) pml_kerne
         T fb0[4], fa0[4];
         load4(FA + 2 * TB, fa0);
         {
-          T w[12];
           load4(FB - 4, v); load4(FB, fb0); load4(FB + 4, u);
 #pragma unroll
           for (int e = 0; e < 4; ++e) { w[e] = v[e]; w[4 + e] = fb0[e]; w[8 + e] = u[e]; }
@@ -954,10 +979,9 @@ __global__ void __launch_bounds__(kPmlThreads, pml_blocks_per_sm<T>()) pml_kerne
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const T pc = pw[3][e];
-          const T lap = (T)270 * s1[e] - (T)27 * s2[e] + (T)2 * s3[e] - (T)1470 * pc;
           const T div = g2[e] + (T)8 * g1[e];
           const T un = (pw[1][e] - pw[5][e]) + (T)8 * (pw[4][e] - pw[2][e]);
-          pnew[e] = ((T)2 * pc - pold[e]) + (a.klap * lap - dz * (pc - pold[e]) + kdiv * div + a.dt2 * f[e]);
+          pnew[e] = ((T)2 * pc - pold[e]) + (a.klap * lap[e] - dz * (pc - pold[e]) + kdiv * div + a.dt2 * f[e]);
           const T fc = fw[2][e];
           fnew[e] = fc - dz * fc - dzr * un;
           fa0[e] += dzr * ua[e];
