@@ -94,9 +94,11 @@ int launch_adjoint_step(Ctx* ctx, int t, int tstep, cudaStream_t s, cudaStream_t
   if (ctx->q_end > ctx->q_begin)
     ARD_CUDA(cudaMemsetAsync(buf + ctx->q_begin, 0, sizeof(T) * (size_t)(ctx->q_end - ctx->q_begin), s));
   if (ctx->n_face_cells > 0) {
-    IfaceAdjArgs<T> ia{buf, ctx->d_ifs, (int)ctx->ifs.size(), ctx->n_face_cells, ctx->d_dct, ctx->d_pml,
-                       ctx->d_mask, lin, lout, (T)ctx->c0, (T)ctx->dh, (T)ctx->dt, ctx->d_cell_iface};
-    ARD_CUDA(launch_dep(iface_adjoint_kernel<T>, grid_for(ctx->n_face_cells, 256, ctx->num_sms * 16), 256, 0, s, ia));
+    IfaceAdjArgs<T> ia{buf, ctx->d_ifs, ctx->d_iface_items, (int)ctx->iface_items.size(), ctx->d_mask, lin, lout,
+                       (T)(ctx->c0 * ctx->c0 / (180.0 * ctx->dh * ctx->dh)), (T)(ctx->dt * ctx->dt)};
+    ARD_CUDA(launch_dep(iface_adjoint_kernel<T>,
+                        grid_for((long long)ctx->iface_items.size(), kIfaceThreads / 32, ctx->num_sms * 16),
+                        kIfaceThreads, 0, s, ia));
     ARD_CUDA(cudaGetLastError());
   }
   const bool fork = !ctx->pml_blocks.empty() && !ctx->dct.empty();

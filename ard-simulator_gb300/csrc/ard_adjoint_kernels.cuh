@@ -32,97 +32,81 @@ template <typename T>
 struct IfaceAdjArgs {
   T* buf;
   const IfaceDev* ifs;
-  int nif;
-  long long total;
-  const DctDev* dct;
-  const PmlDev* pml;
+  const IfaceItem* items;
+  int nitems;
   const unsigned char* masks;
   int lin;    // level of the adjoint PML pressure of step t + 1 (the strip force enters p(t + 1) times dt^2)
   int lout;   // level of the adjoint PML pressure of step t (accumulated)
-  T c0, dh, dt;
-  const int* cell_iface;   // interface of every face cell
+  T k0, dt2;
 };
 
-// Adjoint of the force value that the forward step writes at crossing
-// coordinate c, face coordinates (u, v) of side s.
+// Transpose of iface_kernel, over the same items: every force value the
+// forward step writes (mask bit set) sends its adjoint back through the same
+// 6-point stencil to the three pressure layers on each side that it was
+// computed from.
 template <typename T>
-__device__ __forceinline__ T adj_force(const IfaceAdjArgs<T>& a, int type, const SideDev& s, int c, int u, int v) {
-  if (s.kind == 0) {
-    const DctDev& D = a.dct[s.idx];
-    const int x = type == 0 ? c : u;
-    const int y = type == 0 ? u : (type == 1 ? c : v);
-    const int z = type == 2 ? c : v;
-    const long long o = shell_index(D, x, y, z);
-    return o >= 0 ? a.buf[o - D.fX + D.aX] : (T)0;
-  }
-  const PmlDev& P = a.pml[s.idx];
-  return a.dt * a.dt * a.buf[P.ap[a.lin] + ((long long)c * P.A + v) * P.Bp + u];
-}
-
-// Offset of the adjoint pressure value of crossing coordinate c, face
-// coordinates (u, v) of side s (the cell the forward step read the pressure
-// of).
-template <typename T>
-__device__ __forceinline__ long long adj_pressure_offset(const IfaceAdjArgs<T>& a, int type, const SideDev& s, int c,
-                                                         int u, int v) {
-  if (s.kind == 0) {
-    const DctDev& D = a.dct[s.idx];
-    const int layer = face_layer(c, s.ext);
-    if (type == 0) return D.qX + ((long long)layer * D.d + v) * D.h + u;
-    if (type == 1) return D.qY + ((long long)layer * D.d + v) * D.wp + u;
-    return D.qZ + ((long long)layer * D.h + v) * D.wp + u;
-  }
-  const PmlDev& P = a.pml[s.idx];
-  return P.ap[a.lout] + ((long long)c * P.A + v) * P.Bp + u;
-}
-
-// Transpose of iface_kernel: every force value the forward step writes
-// (mask bit set) sends its adjoint back through the same 6-point stencil to
-// the three pressure layers on each side that it was computed from.
-template <typename T>
-__global__ void __launch_bounds__(256) iface_adjoint_kernel(IfaceAdjArgs<T> a) {
-  grid_dependency_wait();
-  const T C[6][6] = {{0, 0, -2, 2, 0, 0},       {0, -2, 27, -27, 2, 0},     {-2, 27, -270, 270, -27, 2},
-                     {2, -27, 270, -270, 27, -2}, {0, 2, -27, 27, -2, 0},     {0, 0, 2, -2, 0, 0}};
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < a.total;
-       g += (long long)gridDim.x * blockDim.x) {
-    const IfaceDev& I = a.ifs[a.cell_iface[g]];
-    const long long local = g - I.cell0;
-    const int nu = I.u1 - I.u0;
-    const int iu = I.u0 + (int)(local % nu);
-    const int iv = I.v0 + (int)(local / nu);
-    const unsigned mask = a.masks[I.mask + local];
-    const int lu = iu - I.lo.ou, lv = iv - I.lo.ov;
-    const int hu = iu - I.hi.ou, hv = iv - I.hi.ov;
-    const T k = (T)I.absorption * (a.c0 * a.c0) / ((T)180 * a.dh * a.dh);
-    T gl[3] = {0, 0, 0}, gh[3] = {0, 0, 0};
+__global__ void __launch_bounds__(kIfaceThreads) iface_adjoint_kernel(IfaceAdjArgs<T> a) {
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (kIfaceThreads / 32);
+  bool waited = false;
+  for (int i = blockIdx.x * (kIfaceThreads / 32) + (threadIdx.x >> 5); i < a.nitems; i += warps) {
+    const IfaceItem it = a.items[i];
+    const IfaceDev& I = a.ifs[it.iface];
+    const int type = I.type, nu = I.u1 - I.u0;
+    const int u = it.u0 + lane;
+    const bool ok = u < nu;
+    // adjoint forces and pressures: an air side's arrays lie a constant away
+    // from the forward ones, a PML side's strip force entered p(t + 1) of the
+    // same cells times dt^2
+    auto rows = [&](const SideDev& S, bool lo) {
+      const int su = I.u0 + u - S.ou, sv = I.v0 + it.v0 - S.ov;
+      SideRow r = side_row(S, type, lo, su, sv, 0);
+      if (S.kind == 0) {
+        r.f += S.ash;
+        r.p += S.qsh;
+      } else {
+        const long long at = (long long)sv * S.psv + su;
+        r.f = S.ao[a.lin] + at;
+        r.p = S.ao[a.lout] + at;
+      }
+      return r;
+    };
+    SideRow L = rows(I.lo, true), H = rows(I.hi, false);
+    const T ls = I.lo.kind == 0 ? (T)1 : a.dt2, hs = I.hi.kind == 0 ? (T)1 : a.dt2;
+    const bool lself = I.lo.self != 0, hself = I.hi.self != 0;
+    const T k = (T)I.absorption * a.k0;
+    const unsigned char* mk = a.masks + I.mask + (long long)it.v0 * nu + u;
+    if (!waited) {
+      grid_dependency_wait();   // items, descriptors and masks are constants
+      waited = true;
+    }
+    for (int r = 0; r < it.n; ++r) {
+      const unsigned mask = ok ? *mk : 0u;
+      T gl[3] = {0, 0, 0}, gh[3] = {0, 0, 0};
 #pragma unroll
-    for (int m = -3; m < 3; ++m) {
-      if (!(mask & (1u << (m + 3)))) continue;
-      const T fb = m < 0 ? adj_force(a, I.type, I.lo, I.lo.ext + m, lu, lv) : adj_force(a, I.type, I.hi, m, hu, hv);
-      const T g = k * fb;
-      const bool use_lo = m < 0 ? I.lo.self != 0 : true;
-      const bool use_hi = m < 0 ? true : I.hi.self != 0;
+      for (int m = 0; m < 6; ++m) {
+        T fb = 0;
+        if (mask >> m & 1) fb = m < 3 ? ls * a.buf[L.f + m * L.fk] : hs * a.buf[H.f + (m - 3) * H.fk];
+        const T g = k * fb;
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+          if (m >= 3 || lself) gl[n] += g * (T)kIfaceC[m][n];
+          if (m < 3 || hself) gh[n] += g * (T)kIfaceC[m][3 + n];
+        }
+      }
 #pragma unroll
       for (int n = 0; n < 3; ++n) {
-        if (use_lo) gl[n] += g * C[m + 3][n];
-        if (use_hi) gh[n] += g * C[m + 3][3 + n];
+        if (gl[n] != (T)0) atomicAdd(a.buf + L.p + n * L.ps, gl[n]);
+        if (gh[n] != (T)0) atomicAdd(a.buf + H.p + n * H.ps, gh[n]);
       }
-    }
-    // every target offset first, the atomics after them: descriptor fields
-    // read after an atomic through the pool pointer would be loaded again
-    long long ol[3], oh[3];
-#pragma unroll
-    for (int n = 0; n < 3; ++n) {
-      ol[n] = adj_pressure_offset(a, I.type, I.lo, I.lo.ext - 3 + n, lu, lv);
-      oh[n] = adj_pressure_offset(a, I.type, I.hi, n, hu, hv);
-    }
-#pragma unroll
-    for (int n = 0; n < 3; ++n) {
-      if (gl[n] != (T)0) atomicAdd(a.buf + ol[n], gl[n]);
-      if (gh[n] != (T)0) atomicAdd(a.buf + oh[n], gh[n]);
+      mk += nu;
+      L.p += L.pv;
+      L.f += L.fv;
+      H.p += H.pv;
+      H.f += H.fv;
     }
   }
+  if (!waited) grid_dependency_wait();   // no item: still not done before the predecessor
 }
 
 // ---------------------------------------------------------------------------

@@ -129,8 +129,22 @@ struct SideDev {
   int psv;
   int fsv;
   long long fb, fls;
+  // Adjoint: air side, offset of the adjoint shell force from the force and of
+  // the adjoint face pressure from the pressure; PML side, the adjoint
+  // pressure of the first of the side's three layers on its three levels.
+  long long ash, qsh;
+  long long ao[3];
   long long fx, fy, fz;
   int w, h, d, wp;
+};
+
+// A warp's share of an interface: 32 cells along u from u0, n rows from v0
+// (relative to the face range).  A row whose cells an air side's Y layers own
+// (a Z interface's first and last three) is an item of its own, so that the
+// addresses of a lane are linear over an item's rows (side_row).
+struct IfaceItem {
+  int iface;
+  int u0, v0, n;
 };
 
 struct IfaceDev {

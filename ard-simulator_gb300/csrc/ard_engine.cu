@@ -429,9 +429,10 @@ int launch_step(Ctx* ctx, int par, int tstep, cudaStream_t s, cudaStream_t s2, b
   }
   ARD_CUDA(mark(kStageIface));
   if (ctx->n_face_cells > 0) {
-    IfaceArgs<T> ia{buf, ctx->d_ifs, ctx->d_cell_iface, ctx->n_face_cells, ctx->d_mask, par, (T)ctx->c0,
-                    (T)ctx->dh};
-    ARD_CUDA(launch_dep(iface_kernel<T>, grid_for(ctx->n_face_cells, 256, ctx->num_sms * 16), 256, 0, s, ia));
+    IfaceArgs<T> ia{buf, ctx->d_ifs, ctx->d_iface_items, (int)ctx->iface_items.size(), ctx->d_mask, par,
+                    (T)(ctx->c0 * ctx->c0 / (180.0 * ctx->dh * ctx->dh))};
+    ARD_CUDA(launch_dep(iface_kernel<T>, grid_for((long long)ctx->iface_items.size(), kIfaceThreads / 32, ctx->num_sms * 16),
+                        kIfaceThreads, 0, s, ia));
     ARD_CUDA(cudaGetLastError());
   }
   ARD_CUDA(mark(kNumStages));

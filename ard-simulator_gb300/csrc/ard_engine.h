@@ -68,7 +68,7 @@ struct Ctx {
   std::vector<int4> pml_blocks, pml_ablocks;   // plane tiles: forward, adjoint (options.adjoint)
   std::vector<IfaceDev> ifs;
   std::vector<unsigned char> masks;
-  std::vector<int> cell_iface;              // interface of every face cell
+  std::vector<IfaceItem> iface_items;       // the interface kernels' warps
   std::vector<PointDev> srcpts, recpts;
   std::vector<ModalTile> tiles;
   JobList fwd1, fwd2, inv1, inv2;           // two-pass GEMM face transforms
@@ -133,7 +133,7 @@ struct Ctx {
   int4* d_pml_blocks = nullptr;
   int4* d_pml_ablocks = nullptr;
   IfaceDev* d_ifs = nullptr;
-  int* d_cell_iface = nullptr;
+  IfaceItem* d_iface_items = nullptr;
   PointDev* d_srcpts = nullptr;
   PointDev* d_recpts = nullptr;
   ModalTile* d_tiles = nullptr;

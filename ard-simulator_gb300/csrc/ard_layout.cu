@@ -794,15 +794,38 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
         const DctDev& D = ctx->dct[S.idx];
         S.fx = D.fX; S.fy = D.fY; S.fz = D.fZ;
         S.w = D.w; S.h = D.h; S.d = D.d; S.wp = D.wp;
+        S.ash = D.aX - D.fX;
+        S.qsh = D.qX - D.pX;
       } else {
         const PmlDev& P = ctx->pml[S.idx];
         S.fls = (long long)P.A * P.Bp;
         S.fb = P.force - (long long)P.strip0 * S.fls;
         S.fsv = P.Bp;
+        for (int q = 0; q < 3; ++q) S.ao[q] = P.ap[q] + (side == 0 ? S.ext - 3 : 0) * S.fls;
       }
     }
-    for (long long k = 0; k < (long long)(I.u1 - I.u0) * (I.v1 - I.v0); ++k) ctx->cell_iface.push_back((int)ctx->ifs.size());
     ctx->ifs.push_back(I);
+  }
+  {
+    // the interface kernels' warps: one row of 32 cells each while that leaves
+    // SMs without work, up to four rows in large launches (GB300, us per launch
+    // at 1 / 2 / 4 / 8 rows: 0.06 M cells 7.7 / 8.2 / 8.4 / 10.1, 0.13 M 9.2 /
+    // 8.8 / 9.4 / 11.1, 5.9 M 181 / 122 / 101 / 106, 4.1 M 89 / 64 / 56 / 54)
+    long long rows = 0;
+    for (const IfaceDev& I : ctx->ifs) rows += (long long)((I.u1 - I.u0 + 31) / 32) * (I.v1 - I.v0);
+    const int n = (int)std::max(1LL, std::min(4LL, rows / (ctx->num_sms * 16LL)));
+    for (size_t i = 0; i < ctx->ifs.size(); ++i) {
+      const IfaceDev& I = ctx->ifs[i];
+      auto alone = [&](int v) {   // a row on an air side's Y shell
+        for (const SideDev* S : {&I.lo, &I.hi})
+          if (I.type == 2 && S->kind == 0 && face_layer(I.v0 + v - S->ov, S->h) >= 0) return true;
+        return false;
+      };
+      for (int v = 0, k; v < I.v1 - I.v0; v += k) {
+        for (k = 1; !alone(v) && k < n && v + k < I.v1 - I.v0 && !alone(v + k);) ++k;
+        for (int u = 0; u < I.u1 - I.u0; u += 32) ctx->iface_items.push_back(IfaceItem{(int)i, u, v, k});
+      }
+    }
   }
   for (size_t k = 0; k < ctx->pml.size(); ++k) {
     if (pml_iface_count[k] != 1) {
@@ -1072,7 +1095,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
   if ((rc = up(&ctx->d_pml, ctx->pml))) return rc;
   if ((rc = up(&ctx->d_pml_blocks, ctx->pml_blocks))) return rc;
   if ((rc = up(&ctx->d_ifs, ctx->ifs))) return rc;
-  if ((rc = up(&ctx->d_cell_iface, ctx->cell_iface))) return rc;
+  if ((rc = up(&ctx->d_iface_items, ctx->iface_items))) return rc;
   if ((rc = up(&ctx->d_srcpts, ctx->srcpts))) return rc;
   if ((rc = up(&ctx->d_recpts, ctx->recpts))) return rc;
   if ((rc = up(&ctx->d_tiles, ctx->tiles))) return rc;
@@ -1161,7 +1184,7 @@ void free_ctx_device(Ctx* ctx) {
                   ctx->d_inv2d, ctx->d_series,
                   ctx->d_hist, ctx->d_t, ctx->d_adj1_2d, ctx->d_adj2_2d, ctx->d_adjg[0], ctx->d_adjg[1],
                   ctx->d_adjg[2], ctx->d_adjg[3], ctx->d_tb, ctx->d_phist, ctx->d_psum,
-                  ctx->d_cell_iface, ctx->d_mjobs[0], ctx->d_mjobs[1], ctx->d_mjobs[2], ctx->d_mjobs[3],
+                  ctx->d_iface_items, ctx->d_mjobs[0], ctx->d_mjobs[1], ctx->d_mjobs[2], ctx->d_mjobs[3],
                   ctx->d_mjobs[4], ctx->d_mjobs[5], ctx->d_mjobs[6], ctx->d_mjobs[7],
                   ctx->d_err, ctx->d_maps};
   for (void* p : ptrs)
