@@ -138,13 +138,7 @@ int launch_adjoint_step(Ctx* ctx, int t, int tstep, cudaStream_t s, cudaStream_t
     else
       ARD_CUDA(launch_dep(modal_kernel<T, false, true>, mgrid, kModalThreads, msmem, s, ma));
     ARD_CUDA(cudaGetLastError());
-    if (!ctx->srcpts.empty()) {
-      ARD_CUDA(launch_dep(srcgrad_kernel<T>, grid_for((long long)ctx->srcpts.size() * 32, 128, 1 << 30), 128, 0, s,
-                          (const T*)buf, ctx->d_dct, ctx->d_srcpts, (int)ctx->srcpts.size(), ctx->n_src_total,
-                          ab.gsrc, ctx->d_tb, tstep));
-      ARD_CUDA(cudaGetLastError());
-    }
-    if (int rc2 = launch_post_modal<T>(ctx, s, 0, false)) return rc2;
+    if (int rc2 = launch_post_modal_adjoint<T>(ctx, s, ctx->d_tb, tstep, ab.gsrc)) return rc2;
     if (ctx->fused_faces) {
       ARD_CUDA((launch_face<T, true>((long long)ctx->adj2_2d.size() / 2, gx, ctx->f2d_bytes, s, buf, ctx->d_adj2_2d,
                                      ctx->f2d_smem)));
@@ -178,8 +172,12 @@ static __global__ void retreat_counter_kernel(long long* tc, int n) {
 
 // Adjoint steps captured as one CUDA graph: kAdjGraphSteps steps starting at
 // a step t = 5 (mod 6) (the level choices t % 3 and t & 1 repeat every 6
-// steps), the step counter lowered by kAdjGraphSteps at the end.
-constexpr int kAdjGraphSteps = 48;
+// steps), the step counter lowered by kAdjGraphSteps at the end.  The graph
+// holds the call's buffers, so every call captures its own: 12 steps (about
+// 100 nodes) cost 0.8 ms less than 48 and launch as fast (GB300, 192 steps of
+// a small room 8.98 -> 8.22 ms; 6 steps 8.15, but 0.2 ms more for 256 steps of
+// the L-shaped room).
+constexpr int kAdjGraphSteps = 12;
 
 struct AdjGraph {
   cudaGraphExec_t exec = nullptr;
@@ -208,7 +206,7 @@ int capture_adjoint_graph(Ctx* ctx, const AdjBuffers& ab, const HistView& hv, Ad
 }
 
 // Adjoint steps t_hi - 1 down to t_lo: direct launches up to a step t = 5
-// (mod 6), then 48-step graphs, then direct launches for the rest.  Every
+// (mod 6), then 12-step graphs, then direct launches for the rest.  Every
 // launch finds its step as counter - tstep.
 template <typename T>
 int run_backward(Ctx* ctx, long long t_hi, long long t_lo, long long hist_t0, const AdjBuffers& ab,

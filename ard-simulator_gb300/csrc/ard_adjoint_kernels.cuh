@@ -12,7 +12,7 @@
 //   face / GEMM jobs       adjoint of the inverse face transform
 //   modal_kernel<ADJ>      transposed modal recurrence, recorder residual
 //                          injection, source-series gradient partials
-//   srcgrad_kernel         source-series gradient of step t
+//   post_modal_kernel      source-series gradient of step t, partial sums
 //   face / GEMM jobs       adjoint of the forward face transform -> adjoint
 //                          shell force of step t - 1
 #pragma once
@@ -373,29 +373,8 @@ __global__ void __launch_bounds__(256, 4) pml_adjoint_kernel(PmlAdjArgs<T> a) {
 }
 
 // ---------------------------------------------------------------------------
-// Source-series gradient, initial-pressure gradient, counters
+// Initial-pressure gradient, counters
 // ---------------------------------------------------------------------------
-
-// dJ/d series[slot][t] = s_f * (sum of the modal tiles' partials); one warp per source.
-// g is [steps][ld], columns = global source slots.
-template <typename T>
-__global__ void srcgrad_kernel(const T* __restrict__ buf, const DctDev* __restrict__ dct,
-                               const PointDev* __restrict__ srcs, int npts, int ld, double* __restrict__ g,
-                               const long long* tc, int tstep) {
-  grid_dependency_wait();
-  const int lane = threadIdx.x & 31;
-  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (r >= npts) return;
-  const PointDev q = srcs[r];
-  const DctDev& D = dct[q.part];
-  const int local = r - D.src0;
-  const int ntiles = D.ntiles;
-  T s = 0;
-  for (int i = lane; i < ntiles; i += 32) s += buf[D.srcpart + (long long)i * D.nsrc + local];
-  s = warp_sum(s);
-  const long long t = tc[0] - tstep;
-  if (lane == 0) g[t * ld + q.slot] = (double)s * D.sf;
-}
 
 // dJ/dm0 for modes that start at rest (M(-1) = M(-2) = m0):
 // (alpha - a) mu(0) - a mu(1), written unpadded [kz][ky][kx] at `out`.

@@ -470,7 +470,7 @@ int launch_post_modal_range(Ctx* ctx, cudaStream_t s, int tstep, int r_lo, int r
   const int per = nchunks >= wave ? 8 : 0;
   const int sum_blocks = s_total <= 0 ? 0 : (per ? grid_for(nchunks, 1, wave) : grid_for(s_total, 256, wave));
   if (rec_blocks + sum_blocks == 0) return ARD_OK;
-  PostModalArgs<T> a{reinterpret_cast<T*>(ctx->d_buf), ctx->d_dct, ctx->d_recpts, r_lo, nrec, ctx->n_rec_total,
+  PostModalArgs<T> a{reinterpret_cast<T*>(ctx->d_buf), ctx->d_dct, false, ctx->d_recpts, r_lo, nrec, ctx->n_rec_total,
                      ctx->d_hist, ctx->d_t, tstep, ctx->max_steps, rec_blocks, ctx->d_psum + s_lo, s_hi - s_lo,
                      s_first, s_total, per};
   ARD_CUDA(launch_dep(post_modal_kernel<T>, rec_blocks + sum_blocks, 256, 0, s, a));
@@ -481,15 +481,27 @@ int launch_post_modal_range(Ctx* ctx, cudaStream_t s, int tstep, int r_lo, int r
 template int launch_post_modal_range<float>(Ctx*, cudaStream_t, int, int, int, int, int, long long, long long);
 template int launch_post_modal_range<double>(Ctx*, cudaStream_t, int, int, int, int, int, long long, long long);
 
-// Recorder sums (with_recorders) and partial sums of all air partitions in one launch.
+// The adjoint's sums: the source-series gradient of the step (counter `tc`
+// minus tstep) and the partial sums of all air partitions, in one launch.
 template <typename T>
-int launch_post_modal(Ctx* ctx, cudaStream_t s, int tstep, bool with_recorders) {
-  return launch_post_modal_range<T>(ctx, s, tstep, 0, with_recorders ? (int)ctx->recpts.size() : 0, 0,
-                                    (int)ctx->psum.size(), 0, ctx->psum_total);
+int launch_post_modal_adjoint(Ctx* ctx, cudaStream_t s, const long long* tc, int tstep, double* gsrc) {
+  const int n = (int)ctx->srcpts.size(), point_blocks = (n * 32 + 255) / 256;
+  const int wave = ctx->num_sms * 8;
+  const long long nchunks = ctx->psum_total / kSumChunk;
+  const int per = nchunks >= wave ? 8 : 0;
+  const int sum_blocks =
+      ctx->psum_total <= 0 ? 0 : (per ? grid_for(nchunks, 1, wave) : grid_for(ctx->psum_total, 256, wave));
+  if (point_blocks + sum_blocks == 0) return ARD_OK;
+  PostModalArgs<T> a{reinterpret_cast<T*>(ctx->d_buf), ctx->d_dct, true, ctx->d_srcpts, 0, n, ctx->n_src_total,
+                     gsrc, tc, tstep, ctx->max_steps, point_blocks, ctx->d_psum, (int)ctx->psum.size(),
+                     0, ctx->psum_total, per};
+  ARD_CUDA(launch_dep(post_modal_kernel<T>, point_blocks + sum_blocks, 256, 0, s, a));
+  ARD_CUDA(cudaGetLastError());
+  return ARD_OK;
 }
 
-template int launch_post_modal<float>(Ctx*, cudaStream_t, int, bool);
-template int launch_post_modal<double>(Ctx*, cudaStream_t, int, bool);
+template int launch_post_modal_adjoint<float>(Ctx*, cudaStream_t, const long long*, int, double*);
+template int launch_post_modal_adjoint<double>(Ctx*, cudaStream_t, const long long*, int, double*);
 template int launch_step<float>(Ctx*, int, int, cudaStream_t, cudaStream_t, bool, cudaEvent_t*);
 template int launch_step<double>(Ctx*, int, int, cudaStream_t, cudaStream_t, bool, cudaEvent_t*);
 

@@ -189,7 +189,7 @@ void free_graphs(Ctx* ctx);
 int check_guards(Ctx* ctx);
 int check_device_error(Ctx* ctx);
 template <typename T>
-int launch_post_modal(Ctx* ctx, cudaStream_t s, int tstep, bool with_recorders);
+int launch_post_modal_adjoint(Ctx* ctx, cudaStream_t s, const long long* tc, int tstep, double* gsrc);
 template <typename T>
 int launch_post_modal_range(Ctx* ctx, cudaStream_t s, int tstep, int r_lo, int r_hi, int s_lo, int s_hi,
                             long long s_first, long long s_total);

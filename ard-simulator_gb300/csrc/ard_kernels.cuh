@@ -555,9 +555,13 @@ template <typename T>
 struct PostModalArgs {
   T* buf;
   const DctDev* dct;
-  const PointDev* recs;   // all recorders; this launch takes [rec_first, rec_first + nrec)
+  // points read out: the recorders [rec_first, rec_first + nrec) into the
+  // history row of the step, or (adjoint) the sources into the row of the
+  // source-series gradient
+  bool adjoint;
+  const PointDev* recs;
   int rec_first, nrec;
-  int nrec_total;         // row width of the history
+  int nrec_total;         // row width of the history (gradient)
   double* hist;
   const long long* tcount;
   int tstep;
@@ -578,15 +582,25 @@ __global__ void __launch_bounds__(256) post_modal_kernel(PostModalArgs<T> a) {
     const int r = a.rec_first + min(rl, a.nrec - 1);
     const PointDev q = a.recs[r];
     const DctDev& D = a.dct[q.part];
-    const int local_r = r - D.rec0;
+    const int local = r - (a.adjoint ? D.src0 : D.rec0), n = a.adjoint ? D.nsrc : D.nrec;
+    const T* part = a.buf + (a.adjoint ? D.srcpart : D.recpart) + local;
     const int ntiles = D.ntiles;
+    const double scale = a.adjoint ? D.sf : D.si;
     grid_dependency_wait();
     if (rl >= a.nrec) return;
-    T s = 0;
-    for (int i = lane; i < ntiles; i += 32) s += a.buf[D.recpart + (long long)i * D.nrec + local_r];
-    s = warp_sum(s);
-    const long long t = *a.tcount + a.tstep;
-    if (lane == 0 && t < a.max_steps) a.hist[t * a.nrec_total + q.slot] = (double)(s * (T)D.si);
+    T s[4] = {0, 0, 0, 0};   // four loads in flight
+    for (int i = lane; i < ntiles; i += 128)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i + 32 * k < ntiles) s[k] += part[(long long)(i + 32 * k) * n];
+    const T sum = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+    if (lane != 0) return;
+    if (a.adjoint) {
+      a.hist[(*a.tcount - a.tstep) * a.nrec_total + q.slot] = (double)sum * scale;
+    } else {
+      const long long t = *a.tcount + a.tstep;
+      if (t < a.max_steps) a.hist[t * a.nrec_total + q.slot] = (double)(sum * (T)scale);
+    }
     return;
   }
   T* __restrict__ buf = a.buf;
