@@ -28,7 +28,10 @@ namespace ard {
 
 constexpr int kCube = 10;             // cube edge: offsets -5 .. 4 (recorder.cpp:44-52)
 constexpr int kCubeCells = kCube * kCube * kCube;
-constexpr int kCubeRowBlocks = 64;    // rows of stage 1 per block: 8 warps x 8
+constexpr int kCubeLanes = 4;         // lanes of a row in the kx sum
+constexpr int kCubeRows = 128 / kCubeLanes;   // rows of a block
+constexpr int kCubeChunk = 128;       // kx whose basis is staged together
+constexpr int kCubeParts = 4;         // parts of the ky and kz sums
 
 template <typename T>
 struct CubeArgs {
@@ -49,74 +52,124 @@ struct CubeArgs {
   long long max_steps;
 };
 
-// Stage 1: T1[kz][ky][i] = sum_kx M[kz][ky][kx] Ci(kx, x0 + i), one warp per
-// (kz, ky) row of the recorder's partition (Ci^T row x0 + i is contiguous in kx).
+// Each stage is a chain of dependent loads and sums behind the one before, on
+// a few thousand rows: its length is the time, not its bytes.  So the sums are
+// short ones of several threads, added in a fixed order at the end, with the
+// loads of several terms in flight.  GB300, five-partition L-shaped room at 5 cm with
+// its recorders: a step 52.0 -> 38.1 us, the three launches 26 -> 11 us of it.
+
+// Stage 1: T1[kz][ky][i] = sum_kx M[kz][ky][kx] Ci(kx, x0 + i), kCubeLanes
+// lanes per (kz, ky) row of the recorder's partition, four kx of a lane at a
+// time.  The basis (row x0 + i of Ci^T is contiguous in kx) is read from shared
+// memory by four kx too; the ten outputs are added over two shuffles each, where
+// a warp per row took five.
 template <typename T>
-__global__ void __launch_bounds__(256) cube_rows_kernel(CubeArgs<T> a) {
-  grid_dependency_wait();
-  const int rl = blockIdx.x / a.rows_blocks;
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(128) cube_rows_kernel(CubeArgs<T> a) {
+  __shared__ __align__(16) T basis[kCube][kCubeChunk];
+  const int rl = blockIdx.x / a.rows_blocks, tid = threadIdx.x, lane = tid % kCubeLanes;
   const PointDev q = a.recs[a.r_lo + rl];
   const DctDev& D = a.dct[q.part];
-  const int rows = D.d * D.h;
-  const T* ct = a.buf + D.cw + 3LL * D.w * D.w + (long long)(q.x - kCube / 2) * D.w;
-  T* t1 = a.tmp + (long long)(a.r_lo + rl) * a.s1;
-  const int stride = a.rows_blocks * 8;
-  for (int row = (blockIdx.x % a.rows_blocks) * 8 + (threadIdx.x >> 5); row < rows; row += stride) {
-    const T* m = a.buf + D.M[a.par] + (long long)row * D.wp;
-    T acc[kCube];
+  const int w = D.w, rows = D.d * D.h;
+  const int row0 = (blockIdx.x % a.rows_blocks) * kCubeRows, row = row0 + tid / kCubeLanes;
+  const T* ct = a.buf + D.cw + 3LL * w * w + (long long)(q.x - kCube / 2) * w;
+  const T* m = a.buf + D.M[a.par] + (long long)min(row, rows - 1) * D.wp;
+  if (row0 >= rows) return;
+  T acc[kCube];
 #pragma unroll
-    for (int i = 0; i < kCube; ++i) acc[i] = 0;
-    for (int k = lane; k < D.w; k += 32) {
-      const T v = m[k];
+  for (int i = 0; i < kCube; ++i) acc[i] = 0;
+  for (int x0 = 0; x0 < w; x0 += kCubeChunk) {
+    const int n = min(kCubeChunk, w - x0);
+    if (x0) __syncthreads();   // the previous chunk is used up
+    for (int k = tid; k < kCubeChunk; k += 128)
 #pragma unroll
-      for (int i = 0; i < kCube; ++i) acc[i] += v * ct[(long long)i * D.w + k];
+      for (int i = 0; i < kCube; ++i) basis[i][k] = k < n ? ct[(long long)i * w + x0 + k] : (T)0;
+    __syncthreads();
+    if (!x0) grid_dependency_wait();
+#pragma unroll 4
+    for (int k = lane * 4; k < n; k += kCubeLanes * 4) {
+      T v[4];
+      load4(m + x0 + k, v);    // within the row pitch, a multiple of 4
+#pragma unroll
+      for (int e = 1; e < 4; ++e) v[e] = k + e < n ? v[e] : (T)0;
+#pragma unroll
+      for (int i = 0; i < kCube; ++i) {
+        T c[4];
+        load4(&basis[i][k], c);
+        acc[i] += (v[0] * c[0] + v[1] * c[1]) + (v[2] * c[2] + v[3] * c[3]);
+      }
     }
-    T mine = 0;
-#pragma unroll
-    for (int i = 0; i < kCube; ++i) {
-      const T s = warp_sum(acc[i]);
-      if (lane == i) mine = s;
-    }
-    if (lane < kCube) t1[(long long)row * kCube + lane] = mine;
   }
+#pragma unroll
+  for (int i = 0; i < kCube; ++i)
+#pragma unroll
+    for (int o = 1; o < kCubeLanes; o *= 2) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+  T* t1 = a.tmp + (long long)(a.r_lo + rl) * a.s1 + (long long)row * kCube;
+  if (row < rows)
+#pragma unroll
+    for (int i = 0; i < kCube; ++i)
+      if (i % kCubeLanes == lane) t1[i] = acc[i];
+}
+
+// sum_k x[k * sx] * c[k] over the terms of one of kCubeParts parts
+template <typename T>
+__device__ __forceinline__ T cube_part(const T* x, int sx, const T* c, int n, int part) {
+  T s[2] = {0, 0};
+  int k = part;
+  for (; k + 7 * kCubeParts < n; k += 8 * kCubeParts)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e & 1] += x[(long long)(k + e * kCubeParts) * sx] * c[k + e * kCubeParts];
+  for (; k < n; k += kCubeParts) s[0] += x[(long long)k * sx] * c[k];
+  return s[0] + s[1];
+}
+
+// The parts' sums of an output, in a fixed order (thread ji of 128 outputs, part).
+template <typename T>
+__device__ __forceinline__ T cube_add_parts(T s) {
+  __shared__ T part_sum[kCubeParts][128];
+  const int ji = threadIdx.x % 128, part = threadIdx.x / 128;
+  part_sum[part][ji] = s;
+  __syncthreads();
+  T r = part_sum[0][ji];
+#pragma unroll
+  for (int p = 1; p < kCubeParts; ++p) r += part_sum[p][ji];
+  return r;
 }
 
 // Stage 2: T2[kz][j][i] = sum_ky T1[kz][ky][i] Ci(ky, y0 + j); block
-// (recorder, kz), thread j * 10 + i.
+// (recorder, kz), a warp group per part of the sum, thread j * 10 + i.
 template <typename T>
-__global__ void __launch_bounds__(128) cube_cols_kernel(CubeArgs<T> a) {
-  grid_dependency_wait();
+__global__ void __launch_bounds__(128 * kCubeParts) cube_cols_kernel(CubeArgs<T> a) {
   const int rl = blockIdx.x / a.dmax, kz = blockIdx.x % a.dmax;
   const PointDev q = a.recs[a.r_lo + rl];
   const DctDev& D = a.dct[q.part];
-  const int t = threadIdx.x;
-  if (kz >= D.d || t >= kCube * kCube) return;
-  const int j = t / kCube, i = t % kCube;
-  const T* t1 = a.tmp + (long long)(a.r_lo + rl) * a.s1 + (long long)kz * D.h * kCube;
-  const T* ch = a.buf + D.ch + 3LL * D.h * D.h + (long long)(q.y - kCube / 2 + j) * D.h;
-  T s = 0;
-  for (int ky = 0; ky < D.h; ++ky) s += t1[ky * kCube + i] * ch[ky];
-  a.tmp[a.s1 * a.nrec_total + (long long)(a.r_lo + rl) * a.s2 + (long long)kz * kCube * kCube + t] = s;
+  const int h = D.h, ji = threadIdx.x % 128, part = threadIdx.x / 128;
+  const int o = min(ji, kCube * kCube - 1), j = o / kCube, i = o % kCube;
+  const T* t1 = a.tmp + (long long)(a.r_lo + rl) * a.s1 + (long long)kz * h * kCube + i;
+  const T* ch = a.buf + D.ch + 3LL * h * h + (long long)(q.y - kCube / 2 + j) * h;
+  if (kz >= D.d) return;
+  grid_dependency_wait();
+  const T s = cube_add_parts(cube_part(t1, kCube, ch, h, part));
+  if (part == 0 && ji < kCube * kCube)
+    a.tmp[a.s1 * a.nrec_total + (long long)(a.r_lo + rl) * a.s2 + (long long)kz * kCube * kCube + ji] = s;
 }
 
 // Stage 3: cube[k][j][i] = s_i sum_kz T2[kz][j][i] Ci(kz, z0 + k) into the
-// history row of step t (one block of 1000 threads per recorder).
+// history row of step t: block (recorder, k), the threads as in stage 2 (one
+// block of 1000 threads per recorder read all of T2 through one SM).
 template <typename T>
-__global__ void __launch_bounds__(1024) cube_out_kernel(CubeArgs<T> a) {
-  grid_dependency_wait();
-  const int rl = blockIdx.x;
+__global__ void __launch_bounds__(128 * kCubeParts) cube_out_kernel(CubeArgs<T> a) {
+  const int rl = blockIdx.x / kCube, k = blockIdx.x % kCube;
   const PointDev q = a.recs[a.r_lo + rl];
   const DctDev& D = a.dct[q.part];
-  const int o = threadIdx.x;
+  const int d = D.d, ji = threadIdx.x % 128, part = threadIdx.x / 128;
+  const T* t2 = a.tmp + a.s1 * a.nrec_total + (long long)(a.r_lo + rl) * a.s2 + min(ji, kCube * kCube - 1);
+  const T* cd = a.buf + D.cd + 3LL * d * d + (long long)(q.z - kCube / 2 + k) * d;
+  grid_dependency_wait();
   const long long t = *a.tcount + a.tstep;
-  if (o >= kCubeCells || t >= a.max_steps) return;
-  const int k = o / (kCube * kCube), ji = o % (kCube * kCube);
-  const T* t2 = a.tmp + a.s1 * a.nrec_total + (long long)(a.r_lo + rl) * a.s2;
-  const T* cd = a.buf + D.cd + 3LL * D.d * D.d + (long long)(q.z - kCube / 2 + k) * D.d;
-  T s = 0;
-  for (int kz = 0; kz < D.d; ++kz) s += t2[kz * kCube * kCube + ji] * cd[kz];
-  a.hist[(t * a.nrec_total + q.slot) * kCubeCells + o] = (float)(s * (T)D.si);
+  if (t >= a.max_steps) return;
+  const T s = cube_add_parts(cube_part(t2, kCube * kCube, cd, d, part));
+  if (part == 0 && ji < kCube * kCube)
+    a.hist[(t * a.nrec_total + q.slot) * kCubeCells + k * kCube * kCube + ji] = (float)(s * (T)D.si);
 }
 
 template <typename T>
@@ -126,9 +179,9 @@ int launch_cubes(Ctx* ctx, cudaStream_t s, int tstep, int par, int r_lo, int r_h
   CubeArgs<T> a{reinterpret_cast<const T*>(ctx->d_buf), ctx->d_dct, ctx->d_recpts, r_lo, nrec, par,
                 reinterpret_cast<T*>(ctx->d_cube_tmp), ctx->cube_s1, ctx->cube_s2, ctx->cube_row_blocks,
                 ctx->cube_dmax, ctx->d_cube_hist, ctx->n_rec_total, ctx->d_t, tstep, ctx->max_steps};
-  ARD_CUDA(launch_dep(cube_rows_kernel<T>, (long long)nrec * a.rows_blocks, 256, 0, s, a));
-  ARD_CUDA(launch_dep(cube_cols_kernel<T>, (long long)nrec * a.dmax, 128, 0, s, a));
-  ARD_CUDA(launch_dep(cube_out_kernel<T>, nrec, 1024, 0, s, a));
+  ARD_CUDA(launch_dep(cube_rows_kernel<T>, (long long)nrec * a.rows_blocks, 128, 0, s, a));
+  ARD_CUDA(launch_dep(cube_cols_kernel<T>, (long long)nrec * a.dmax, 128 * kCubeParts, 0, s, a));
+  ARD_CUDA(launch_dep(cube_out_kernel<T>, (long long)nrec * kCube, 128 * kCubeParts, 0, s, a));
   ARD_CUDA(cudaGetLastError());
   return ARD_OK;
 }
@@ -419,7 +472,7 @@ extern "C" int ard_record_neighbourhoods(ard_ctx* c, int32_t enable) {
   const int nr = ctx->n_rec_total;
   ctx->cube_s1 = rows * kCube;
   ctx->cube_s2 = dmax * kCube * kCube;
-  ctx->cube_row_blocks = (int)std::max(1LL, (rows + kCubeRowBlocks - 1) / kCubeRowBlocks);
+  ctx->cube_row_blocks = (int)((rows + kCubeRows - 1) / kCubeRows);
   ctx->cube_dmax = (int)dmax;
   const size_t es = elem_size(ctx);
   const size_t hist_bytes = sizeof(float) * (size_t)ctx->max_steps * nr * kCubeCells;
