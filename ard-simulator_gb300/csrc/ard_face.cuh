@@ -82,29 +82,44 @@ inline FaceSmem face_smem(const Face2DJob& J, int half, bool inverse) {
   return m;
 }
 
+// Division by a value of the job: i / d = umulhi(i + 1, floor((2^32 - 1) / d)),
+// exact for 0 <= i, (i + 1) d <= 2^32.  The kernel's loops split their flat
+// index by such values all the time; with the compiler's division that was
+// half of its instructions.
+struct FaceDiv {
+  unsigned m;
+  int d;
+  __device__ __forceinline__ explicit FaceDiv(int v) : m(0xffffffffu / (unsigned)v), d(v) {}
+  __device__ __forceinline__ int split(int i, int& rem) const {
+    const int q = (int)__umulhi((unsigned)i + 1u, m);
+    rem = i - q * d;
+    return q;
+  }
+};
+
 // One half-size product per unit: W[u][r][c] = sum_k L[u][r][k] R[u][k][c] for
 // r < rows, c < 4 nq, k < K (a multiple of 4; operands are zero past their
 // extent).  A thread owns MR rows x 4 columns; its rows are rg apart, so the
 // rows that a warp loads together are consecutive.
 template <typename T, int MR, typename LOf, typename ROf, typename Out>
-__device__ __forceinline__ void face_product(int units, int rows, int K, int nq, int lp, int rp, LOf l_of, ROf r_of,
-                                             Out out) {
-  const int rg = (rows + MR - 1) / MR;
-  for (int tile = threadIdx.x; tile < units * rg * nq; tile += kFaceThreads) {
-    const int ct = tile % nq, rest = tile / nq, rt = rest % rg, u = rest / rg;
+__device__ __forceinline__ void face_product(int units, int rows, int K, const FaceDiv& nq, int lp, int rp, LOf l_of,
+                                             ROf r_of, Out out) {
+  const FaceDiv rg((rows + MR - 1) / MR);
+  for (int tile = threadIdx.x; tile < units * rg.d * nq.d; tile += kFaceThreads) {
+    int ct, rt;
+    const int u = rg.split(nq.split(tile, ct), rt);
     const T* L = l_of(u) + rt * lp;
     const T* Rr = r_of(u) + 4 * ct;
     int lo[MR];
 #pragma unroll
-    for (int i = 0; i < MR; ++i) lo[i] = (rt + i * rg < rows ? i * rg : 0) * lp;
-    T acc[MR][4];
+    for (int i = 0; i < MR; ++i) lo[i] = (rt + i * rg.d < rows ? i * rg.d : 0) * lp;
+    Pair<T> acc[MR][2];
 #pragma unroll
-    for (int i = 0; i < MR; ++i)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[i][c] = 0;
+    for (int i = 0; i < MR; ++i) acc[i][0] = acc[i][1] = {0, 0};
 #pragma unroll 2
     for (int k = 0; k < K; k += 4) {
-      T l[MR][4], r[4][4];
+      T l[MR][4];
+      Pair<T> r[4][2];
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) load4(Rr + (k + kk) * rp, r[kk]);
 #pragma unroll
@@ -114,11 +129,14 @@ __device__ __forceinline__ void face_product(int units, int rows, int K, int nq,
 #pragma unroll
         for (int i = 0; i < MR; ++i)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) acc[i][c] += l[i][kk] * r[kk][c];
+          for (int c = 0; c < 2; ++c) acc[i][c] = fma2(dup2(l[i][kk]), r[kk][c], acc[i][c]);
     }
 #pragma unroll
     for (int i = 0; i < MR; ++i)
-      if (rt + i * rg < rows) out(u, rt + i * rg, 4 * ct, acc[i]);
+      if (rt + i * rg.d < rows) {
+        const T v[4] = {acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y};
+        out(u, rt + i * rg.d, 4 * ct, v);
+      }
   }
 }
 
@@ -153,12 +171,13 @@ __device__ __forceinline__ void load_quad(const T* p, int n, bool vec, T (&v)[4]
 // columns each (INV true).
 //
 // Small launches (one room) are bound by the chain load - product - product -
-// store of one block, large ones (batches) by the shared-memory loads of the
-// products.  Layers go through registers once (folded or sorted by parity on
-// the way), tables by cp.async underneath.  GB300, both directions of a step,
+// store of one block, large ones (batches) by instruction issue (47 %) and the
+// barriers between the phases.  Layers go through registers once (folded or
+// sorted by parity on the way), tables by cp.async underneath; indexes are
+// split by multiplication (FaceDiv) and the products run on packed FP32 pairs.  GB300, both directions of a step,
 // against full-length products with rows split over a cluster: one 100^3 room
-// 25 -> 19 us, the L-shaped room of 1.9 M cells 51 -> 42 us, 128 scenes 714 ->
-// 485 us; FP64 (0.24 M cells) 213 -> 129 us.  Rounding improves with the
+// 25 -> 17 us, the L-shaped room of 1.9 M cells 51 -> 38 us, 128 scenes 714 ->
+// 435 us (485 us with compiled divisions, 449 us with scalar products); FP64 (0.24 M cells) 213 -> 129 us.  Rounding improves with the
 // shorter sums.
 template <typename T, bool INV>
 __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ buf, const Face2DJob* __restrict__ jobs,
@@ -179,23 +198,26 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
     const int fp = face_pitch(U), ap = face_pitch(V);
     const int nq = (s.nc + 3) >> 2, ncp = 4 * nq;
     const int npu = s.npu, units = s.no * 2 * npu;   // unit = (out 2 + pv) npu + pu
+    const int su = npu - 1;                          // npu is 1 or 2: u / npu = u >> su, u % npu = u & su
+    const FaceDiv dq(nq);
     __syncthreads();   // the previous job is done with shared memory
     // ---- tables (zero-padded rows, always 16-byte aligned) ----
-    for (int i = tid; i < 2 * hv * (hv4 >> 2); i += kFaceThreads) {
-      const int row = i / (hv4 >> 2), q = i - row * (hv4 >> 2);
+    const FaceDiv dv(hv4 >> 2), du(hu4);
+    for (int i = tid; i < 2 * hv * dv.d; i += kFaceThreads) {
+      int q;
+      const int row = dv.split(i, q);
       cp_async4(As + row * ap + 4 * q, buf + J.tabA + (long long)row * hv4 + 4 * q, true);
     }
     for (int i = tid; i < npu * hu4 * nq; i += kFaceThreads) {
-      const int c = i % nq, rest = i / nq, j = rest % hu4, p = rest / hu4;
+      int c, j;
+      const int p = du.split(dq.split(i, c), j);
       const bool ok = j < hu && s.c0 + 4 * c < hu4;
       cp_async4(Bs + (p * hu4 + j) * ncp + 4 * c,
                 buf + J.tabB + (ok ? ((long long)(s.pu0 + p) * hu + j) * hu4 + s.c0 + 4 * c : 0), ok);
     }
     cp_async_commit();
-    for (int i = tid; i < units * (hv4 - hv) * ncp; i += kFaceThreads) {   // rows past the half length read as zero
-      const int u = i / ((hv4 - hv) * ncp);
-      Ts[(u * hv4 + hv) * ncp + i - u * (hv4 - hv) * ncp] = (T)0;
-    }
+    for (int i = tid; i < (hv4 - hv) * ncp; i += kFaceThreads)   // rows past the half length read as zero
+      for (int u = 0; u < units; ++u) Ts[(u * hv4 + hv) * ncp + i] = (T)0;
     if (!waited) {
       grid_dependency_wait();
       waited = true;
@@ -203,11 +225,12 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
     // ---- the layers, combined and folded (or sorted by parity) ----
     const T* X[2] = {buf + J.in0, buf + J.in1};
     const bool al = ((J.in0 | J.in1 | ld) & 3) == 0;
-    const int nqu = hu4 >> 2;
     if constexpr (!INV) {
       const bool alr = al && (U & 3) == 0;
-      for (int i = tid; i < hv * nqu; i += kFaceThreads) {
-        const int r = i / nqu, q = i - r * nqu, r2 = V - 1 - r;
+      const FaceDiv dqu(hu4 >> 2);
+      for (int i = tid; i < hv * dqu.d; i += kFaceThreads) {
+        int q;
+        const int r = dqu.split(i, q), r2 = V - 1 - r;
         const int n = min(4, hu - 4 * q);
         T d[2][2][4], m[2][2][4];   // [layer][row r, row r2]: direct, mirrored along U
 #pragma unroll
@@ -259,9 +282,10 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
       }
     } else {
       // quads of two half-columns: rows kv (zeros past V), columns 4 q .. 4 q + 3
-      const int nq2 = hu4 >> 1;
-      for (int i = tid; i < 2 * hv * nq2; i += kFaceThreads) {
-        const int kv = i / nq2, q = i - kv * nq2;
+      const FaceDiv dq2(hu4 >> 1);
+      for (int i = tid; i < 2 * hv * dq2.d; i += kFaceThreads) {
+        int q;
+        const int kv = dq2.split(i, q);
         const int n = kv < V ? U - 4 * q : 0;
         T x0[4], x1[4];
         load_quad(X[0] + (long long)kv * ld + 4 * q, n, al, x0);
@@ -284,20 +308,20 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
     __syncthreads();
     // ---- T = F B ----
     auto f_of = [&](int u) { return Fs + u * hv * fp; };
-    auto b_of = [&](int u) { return Bs + (u % npu) * hu4 * ncp; };
+    auto b_of = [&](int u) { return Bs + (u & su) * hu4 * ncp; };
     auto to_t = [&](int u, int r, int c, const T (&v)[4]) { store4(Ts + (u * hv4 + r) * ncp + c, v); };
     const bool wide = units * ((hv + 3) >> 2) * nq >= kFaceThreads / 2;
-    if (wide) face_product<T, 4>(units, hv, hu4, nq, fp, ncp, f_of, b_of, to_t);
-    else      face_product<T, 2>(units, hv, hu4, nq, fp, ncp, f_of, b_of, to_t);
+    if (wide) face_product<T, 4>(units, hv, hu4, dq, fp, ncp, f_of, b_of, to_t);
+    else      face_product<T, 2>(units, hv, hu4, dq, fp, ncp, f_of, b_of, to_t);
     __syncthreads();
     if (it + (int)gridDim.x >= entries) grid_launch_dependents();
     // ---- O = A T ----
     const T scale = (T)J.scale;
-    auto a_of = [&](int u) { return As + (u / npu % 2) * hv * ap; };
+    auto a_of = [&](int u) { return As + (u >> su & 1) * hv * ap; };
     auto t_of = [&](int u) { return Ts + u * hv4 * ncp; };
     if constexpr (!INV) {
       auto to_out = [&](int u, int r, int c, const T (&v)[4]) {
-        const int pu = s.pu0 + u % npu, pv = u / npu % 2, o = s.o0 + u / (2 * npu);
+        const int pu = s.pu0 + (u & su), pv = u >> su & 1, o = s.o0 + (u >> su >> 1);
         const int kv = 2 * r + pv, ku = 2 * (s.c0 + c) + pu;
         if (kv >= V) return;
         T* p = buf + (o ? J.out1 : J.out0) + (long long)kv * ld + ku;
@@ -305,16 +329,18 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
         for (int e = 0; e < 4; ++e)
           if (c + e < s.nc && ku + 2 * e < U) p[2 * e] = v[e] * scale;
       };
-      if (wide) face_product<T, 4>(units, hv, hv4, nq, ap, ncp, a_of, t_of, to_out);
-      else      face_product<T, 2>(units, hv, hv4, nq, ap, ncp, a_of, t_of, to_out);
+      if (wide) face_product<T, 4>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_out);
+      else      face_product<T, 2>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_out);
     } else {
       auto to_o = [&](int u, int r, int c, const T (&v)[4]) { store4(Fs + (u * hv + r) * ncp + c, v); };
-      if (wide) face_product<T, 4>(units, hv, hv4, nq, ap, ncp, a_of, t_of, to_o);
-      else      face_product<T, 2>(units, hv, hv4, nq, ap, ncp, a_of, t_of, to_o);
+      if (wide) face_product<T, 4>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_o);
+      else      face_product<T, 2>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_o);
       __syncthreads();
       // ---- the quadrants' butterfly ----
+      const FaceDiv dc(ncp), dr(hv);
       for (int i = tid; i < s.no * hv * ncp; i += kFaceThreads) {
-        const int c = i % ncp, rest = i / ncp, r = rest % hv, o = rest / hv;
+        int c, r;
+        const int o = dr.split(dc.split(i, c), r);
         const int u = s.c0 + c, u2 = U - 1 - u, r2 = V - 1 - r;
         if (c >= s.nc || u >= hu) continue;
         const T* q = Fs + (o * 4 * hv + r) * ncp + c;   // units (pv, pu) = 0 .. 3, hv rows apart

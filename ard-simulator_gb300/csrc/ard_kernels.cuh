@@ -70,6 +70,49 @@ __device__ __forceinline__ void store4(double* p, const double (&r)[4]) {
   reinterpret_cast<double2*>(p)[1] = make_double2(r[2], r[3]);
 }
 
+// ---- pairs of elements: packed FP32 arithmetic (one instruction for two
+// IEEE-rounded results, sm_100 and later), two scalar operations for FP64 ----
+template <typename T>
+struct alignas(2 * sizeof(T)) Pair {
+  T x, y;
+};
+__device__ __forceinline__ unsigned long long& pair_bits(Pair<float>& p) { return reinterpret_cast<unsigned long long&>(p); }
+__device__ __forceinline__ Pair<float> fma2(Pair<float> a, Pair<float> b, Pair<float> c) {
+  Pair<float> r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(pair_bits(r)) : "l"(pair_bits(a)), "l"(pair_bits(b)), "l"(pair_bits(c)));
+  return r;
+}
+__device__ __forceinline__ Pair<float> mul2(Pair<float> a, Pair<float> b) {
+  Pair<float> r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(pair_bits(r)) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+  return r;
+}
+__device__ __forceinline__ Pair<float> add2(Pair<float> a, Pair<float> b) {
+  Pair<float> r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(pair_bits(r)) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+  return r;
+}
+__device__ __forceinline__ Pair<double> fma2(Pair<double> a, Pair<double> b, Pair<double> c) {
+  return {fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)};
+}
+__device__ __forceinline__ Pair<double> mul2(Pair<double> a, Pair<double> b) { return {a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ Pair<double> add2(Pair<double> a, Pair<double> b) { return {a.x + b.x, a.y + b.y}; }
+template <typename T>
+__device__ __forceinline__ Pair<T> dup2(T v) { return {v, v}; }
+// four consecutive elements as two pairs
+template <typename T>
+__device__ __forceinline__ void load4(const T* p, Pair<T> (&r)[2]) {
+  T v[4];
+  load4(p, v);
+  r[0] = {v[0], v[1]};
+  r[1] = {v[2], v[3]};
+}
+template <typename T>
+__device__ __forceinline__ void store4(T* p, const Pair<T> (&r)[2]) {
+  const T v[4] = {r[0].x, r[0].y, r[1].x, r[1].y};
+  store4(p, v);
+}
+
 // ---- asynchronous global -> shared copies (cp.async, L2-cached) ----
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
