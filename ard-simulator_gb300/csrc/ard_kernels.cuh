@@ -580,6 +580,7 @@ inline cudaError_t configure_face_gemm() {
 // job's elements occupy [first, first + count) of the launch's index space,
 // first a multiple of kSumChunk.
 constexpr int kSumChunk = 2048;
+constexpr int kSumBlocksPerSM = 5;   // resident blocks of the sums (8: 83 us, 5: 78 us, 4: 79 us for 15 M sums)
 struct SumJob {
   long long base;     // slab 0
   long long count;    // elements per slab
@@ -618,7 +619,7 @@ struct PostModalArgs {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256) post_modal_kernel(PostModalArgs<T> a) {
+__global__ void __launch_bounds__(256, kSumBlocksPerSM) post_modal_kernel(PostModalArgs<T> a) {
   if ((int)blockIdx.x < a.rec_blocks) {
     const int lane = threadIdx.x & 31;
     const int rl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
