@@ -289,8 +289,15 @@ __global__ void __launch_bounds__(256, 4) pml_adjoint_kernel(PmlAdjArgs<T> a) {
       T g = 0;
       if (inside && !s_abort) {
         T lx = 0;
+        // the weights sum to zero: in FP32 taps minus the centre, so that the rounding
+        // is that of the differences (as in pml_kernel; FP64 is bound by its operations)
+        const T x0 = xw[3];
 #pragma unroll
-        for (int m = 0; m < 7; ++m) lx += c7[m] * (xw[m] + Xs[(ta + m) * PW + tb + 4] + Xs[(ta + 3) * PW + tb + 1 + m]);
+        for (int m = 0; m < 7; ++m) {
+          const T xa = Xs[(ta + m) * PW + tb + 4], xb = Xs[(ta + 3) * PW + tb + 1 + m];
+          if (sizeof(T) == 8) lx += c7[m] * (xw[m] + xa + xb);
+          else if (m != 3) lx += c7[m] * ((xw[m] - x0) + (xa - x0) + (xb - x0));
+        }
         T dnx = 0, dax = 0, dbx = 0, dnz = 0, daf = 0, dbf = 0;
 #pragma unroll
         for (int m = 0; m < 5; ++m) {
@@ -306,10 +313,9 @@ __global__ void __launch_bounds__(256, 4) pml_adjoint_kernel(PmlAdjArgs<T> a) {
         dnz *= r12; daf *= r12; dbf *= r12;
         const long long I = l * lstride + col;
         const T zn = zeta[l];
-        const T x0 = xw[3];
         const T fa0 = FA[(ta + 2) * TB + tb], fb0 = FB[ta * PW + tb + 4];
-        O[I] = o0 + (T)2 * x0 + dt2 * a.c0 * a.c0 * lx - dt * zn * x0 + (dt * zn - (T)1) * y0 + dt * dnz -
-               dt * zn * (daf + dbf);
+        // 2 X - Y as X + (X - Y): the small terms meet the difference first
+        O[I] = x0 + ((x0 - y0) + (dt2 * a.c0 * a.c0 * lx - dt * zn * (x0 - y0) + dt * dnz - dt * zn * (daf + dbf))) + o0;
         Y[I] = 0;
         Fn_o[I] = ((T)1 - dt * zn) * fn0 - dt2 * dnx;
         Fa_o[I] = fa0 - dt2 * dax;
