@@ -20,9 +20,10 @@
 //                       layers / PML strips (owner masks resolve overlapping
 //                       strips in the reference's list order)
 // The air partitions' kernels (face, modal, sums) launch once per air group
-// (up to two groups on two streams).  Every step kernel starts with
-// grid_dependency_wait: the host launches them with programmatic stream
-// serialization.  xform_gemm_kernel (register-staged GEMM) serves the dense
+// (up to two groups on two streams).  The host launches the step kernels with
+// programmatic stream serialization; each loads its constants and then waits
+// (grid_dependency_wait) before it touches what earlier kernels write.
+// xform_gemm_kernel (register-staged GEMM) serves the dense
 // whole-field transforms of the readouts and the initial pressure.
 #pragma once
 

@@ -174,7 +174,7 @@ bool balance_face_jobs(std::vector<Face2DJob>* jobs, int slots) {
       b.which = 2;
       jobs->push_back(b);
       ctas += 1;
-    } else if (!J.split && J.V > 1) {   // rows split over the cluster
+    } else if (!J.split && J.V > 1) {   // two halves (face_shape)
       J.split = 1;
       ctas += 1;
     } else {

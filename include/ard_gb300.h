@@ -169,7 +169,7 @@ typedef struct ard_options {
   int32_t use_graphs;    /* capture step sequences in CUDA graphs (default 1) */
   int32_t device;        /* CUDA device ordinal */
   int32_t autotune;      /* nonzero: build each candidate layout (modal tile counts,
-                            lanes per ky row, fused or GEMM face transforms), time
+                            fused or two-pass face transforms), time
                             128 steps of each, keep the fastest (default 0) */
   int32_t arithmetic;    /* ARD_ARITH_ACCURATE (default) or ARD_ARITH_REFERENCE */
   int32_t adjoint;       /* nonzero: allocate the adjoint state (needed by ard_adjoint) */
