@@ -172,7 +172,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, 4) pml_adjoint_kernel(PmlAdjArgs<T> a) {
   grid_dependency_wait();
   using S = PmlAdjStage<T>;
-  constexpr int TA = kPmlTA, TB = kPmlTB, PW = S::PW;
+  constexpr int TB = kPmlTB, PW = S::PW;
   __shared__ __align__(128) unsigned char stage[2][S::bytes];
   __shared__ uint64_t bar[2];
   __shared__ volatile int s_abort;

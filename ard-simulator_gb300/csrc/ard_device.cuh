@@ -153,7 +153,6 @@ struct IfaceDev {
   SideDev lo, hi;         // left/top/front and right/bottom/back
   double absorption;
   long long mask;         // [cells] 6-bit write masks (bit m+3)
-  long long cell0;        // first global face-cell index of this interface
 };
 
 // One batched 1D transform as a small GEMM, Out[m][nn] (row pitch ld):

@@ -750,7 +750,6 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
       return ARD_ERR_RANGE;
     }
     I.mask = (long long)ctx->masks.size();
-    I.cell0 = ctx->n_face_cells;
     for (int v = I.v0; v < I.v1; ++v)
       for (int u = I.u0; u < I.u1; ++u) {
         unsigned char bits = 0;
