@@ -523,9 +523,17 @@ int launch_steps_direct(Ctx* ctx, int n, cudaStream_t s) {
 }
 
 // Captures n steps from parity `par` into a graph: the three streams forked
-// and joined per step, the step counter advanced at the end.
+// and joined per step, the step counter advanced at the end.  The calling
+// thread's capture mode is relaxed meanwhile: while any stream of the process
+// is captured in the global mode (a caller's own graph), instantiating a graph
+// would be refused otherwise and the caller's capture would be lost with it.
 static int capture_steps(Ctx* ctx, int n, int par, cudaGraphExec_t* exec) {
   if (*exec) return ARD_OK;
+  struct RelaxedCaptureMode {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
   cudaGraph_t g = nullptr;
   ARD_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   int rc = ARD_OK;
@@ -539,7 +547,11 @@ static int capture_steps(Ctx* ctx, int n, int par, cudaGraphExec_t* exec) {
   if (e != cudaSuccess) { ctx->err = std::string("graph capture: ") + cudaGetErrorString(e); return ARD_ERR_CUDA; }
   e = cudaGraphInstantiate(exec, g, 0);
   cudaGraphDestroy(g);
-  if (e != cudaSuccess) { ctx->err = std::string("graph instantiate: ") + cudaGetErrorString(e); return ARD_ERR_CUDA; }
+  if (e != cudaSuccess) {
+    *exec = nullptr;
+    ctx->err = std::string("graph instantiate: ") + cudaGetErrorString(e);
+    return ARD_ERR_CUDA;
+  }
   return ARD_OK;
 }
 
