@@ -73,7 +73,10 @@ __global__ void __launch_bounds__(128) cube_rows_kernel(CubeArgs<T> a) {
   const int row0 = (blockIdx.x % a.rows_blocks) * kCubeRows, row = row0 + tid / kCubeLanes;
   const T* ct = a.buf + D.cw + 3LL * w * w + (long long)(q.x - kCube / 2) * w;
   const T* m = a.buf + D.M[a.par] + (long long)min(row, rows - 1) * D.wp;
-  if (row0 >= rows) return;
+  if (row0 >= rows) {   // a recorder of a smaller partition than the launch's largest
+    grid_dependency_wait();
+    return;
+  }
   T acc[kCube];
 #pragma unroll
   for (int i = 0; i < kCube; ++i) acc[i] = 0;
@@ -146,8 +149,8 @@ __global__ void __launch_bounds__(128 * kCubeParts) cube_cols_kernel(CubeArgs<T>
   const int o = min(ji, kCube * kCube - 1), j = o / kCube, i = o % kCube;
   const T* t1 = a.tmp + (long long)(a.r_lo + rl) * a.s1 + (long long)kz * h * kCube + i;
   const T* ch = a.buf + D.ch + 3LL * h * h + (long long)(q.y - kCube / 2 + j) * h;
-  if (kz >= D.d) return;
   grid_dependency_wait();
+  if (kz >= D.d) return;
   const T s = cube_add_parts(cube_part(t1, kCube, ch, h, part));
   if (part == 0 && ji < kCube * kCube)
     a.tmp[a.s1 * a.nrec_total + (long long)(a.r_lo + rl) * a.s2 + (long long)kz * kCube * kCube + ji] = s;
