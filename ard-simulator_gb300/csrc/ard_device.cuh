@@ -63,7 +63,7 @@ struct DctDev {
   long long PX, PY, PZ;
   long long RX, RY, RZ;
   long long tmpX, tmpY, tmpZ;
-  long long cw, ch, cd;    // cosine tables of extents w, h, d: C, Ci, C^T, Ci^T (n*n each)
+  long long cw, ch, cd;    // cosine tables of extents w, h, d: C, Ci, Ci^T (n*n each)
   long long recpart;       // [ntiles][nrec]
   long long srcpart;       // [ntiles][nsrc] (adjoint: source-gradient partials)
   long long AM[2];         // adjoint of the modal levels
@@ -104,7 +104,6 @@ struct PmlDev {
   long long force;        // [3][A][Bp]
   long long ap[3];         // adjoint of p (three rotating levels)
   long long aphn[2], apha[2], aphb[2];
-  long long aforce;        // adjoint of the strip force [3][A][Bp]
   long long zeta;         // [L] damping profile (scaled)
   long long n;            // L*A*Bp elements (padding columns stay zero)
   long long hoff;         // offset of the slab inside each all-slab region (p, phi: same for all eight)

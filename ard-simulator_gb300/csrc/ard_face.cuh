@@ -12,7 +12,6 @@
 namespace ard {
 
 constexpr int kFaceThreads = 256;
-constexpr int kFaceCols = 16;        // columns of a quadrant that a job takes (a 32-column slab of the layer)
 
 // Half length of a transform, its padded form, and the row pitch of staged
 // operands: 4 mod 8 elements, so that consecutive rows start in distinct
@@ -71,14 +70,13 @@ __host__ __device__ inline FaceShape face_shape(const Face2DJob& J, int half, bo
 }
 inline FaceSmem face_smem(const Face2DJob& J, int half, bool inverse) {
   const FaceShape s = face_shape(J, half, inverse);
-  const int hv = face_half(J.V), hu = face_half(J.U), nc4 = (s.nc + 3) & ~3, units = s.no * 2 * s.npu;
+  const int hv = face_half(J.V), nc4 = (s.nc + 3) & ~3, units = s.no * 2 * s.npu;
   FaceSmem m;
   m.f = units * hv * face_pitch(J.U);
   if (inverse) m.f = std::max(m.f, units * hv * nc4);
   m.a = 2 * hv * face_pitch(J.V);
   m.b = s.npu * face_half4(J.U) * nc4;
   m.t = units * face_half4(J.V) * nc4;
-  (void)hu;
   return m;
 }
 

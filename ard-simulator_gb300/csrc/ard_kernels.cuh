@@ -616,7 +616,7 @@ struct PostModalArgs {
   int njobs;
   long long first;
   long long total;        // a multiple of kSumChunk
-  int per;                // elements per thread: 1, 2, 4 or 8 (chunked), 0: one element per thread
+  bool chunked;           // chunks of kSumChunk elements; else one element per thread
 };
 
 template <typename T>
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(256, kSumBlocksPerSM) post_modal_kernel(PostMo
   // of the index space, so a chunk lies in one job; a thread sums 8 elements
   // (256 apart) over the job's slabs, slab by slab in order
   const long long nb = (long long)gridDim.x - a.rec_blocks;
-  if (a.per == 0) {
+  if (!a.chunked) {
     // small launches: one element per thread, all its slabs in flight at once
     for (long long g = ((long long)blockIdx.x - a.rec_blocks) * blockDim.x + threadIdx.x; g < a.total;
          g += nb * blockDim.x) {
@@ -688,14 +688,8 @@ __global__ void __launch_bounds__(256, kSumBlocksPerSM) post_modal_kernel(PostMo
     }
     return;
   }
-  // work items: a chunk in kSumChunk / (256 per) parts of 256 per elements,
-  // `per` (1, 2, 4 or 8) elements per thread, 256 apart
-  const int per = a.per;
-  const int parts = kSumChunk / (256 * per);
-  const long long nitems = a.total / kSumChunk * parts;
-  for (long long item = (long long)blockIdx.x - a.rec_blocks; item < nitems; item += nb) {
-    const long long ch = item / parts;
-    const int part = (int)(item - ch * parts);
+  const long long nchunks = a.total / kSumChunk;
+  for (long long ch = (long long)blockIdx.x - a.rec_blocks; ch < nchunks; ch += nb) {
     const long long gg = a.first + ch * kSumChunk;   // first element of the chunk among all sum jobs
     int lo = 0, hi = a.njobs - 1;
     while (lo < hi) {
@@ -703,7 +697,7 @@ __global__ void __launch_bounds__(256, kSumBlocksPerSM) post_modal_kernel(PostMo
       if ((cached ? sfirst[mid] : a.jobs[mid].first) <= gg) lo = mid; else hi = mid - 1;
     }
     const SumJob J = a.jobs[lo];
-    const long long e0 = gg - J.first + (long long)part * 256 * per;
+    const long long e0 = gg - J.first;
     T* p = buf + J.base + e0;
     constexpr int kPer = kSumChunk / 256;
     bool ok[kPer];
@@ -711,7 +705,7 @@ __global__ void __launch_bounds__(256, kSumBlocksPerSM) post_modal_kernel(PostMo
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       const int idx = (int)threadIdx.x + 256 * i;
-      ok[i] = i < per && e0 + idx < J.count;
+      ok[i] = e0 + idx < J.count;
       v[i] = ok[i] ? p[idx] : (T)0;
     }
 #pragma unroll 2
@@ -1222,10 +1216,10 @@ static __global__ void advance_time_kernel(long long* tcount, int n) {
 
 // ---- setup kernels (FP64 arithmetic) ----
 
-// Per extent n, four n*n tables: C[k][j] = 2 cos(pi (j + 1/2) k / n) (the
+// Per extent n, three n*n tables: C[k][j] = 2 cos(pi (j + 1/2) k / n) (the
 // REDFT10 matrix), the REDFT01 matrix Ci[k][j] = C[k][j] with row k = 0
-// halved (REDFT01 weights X_0 by 1, the others by 2), and the transposes of
-// both (row-contiguous access for the fused face transforms).
+// halved (REDFT01 weights X_0 by 1, the others by 2), and the transpose of Ci
+// (contiguous along k, as the neighbourhood sums read it).
 template <typename T>
 __global__ void cos_table_kernel(T* buf, long long off, int n) {
   const long long nn = (long long)n * n;
@@ -1234,11 +1228,9 @@ __global__ void cos_table_kernel(T* buf, long long off, int n) {
     const long long q = ((long long)(2 * j + 1) * k) % (4LL * n);  // argument reduced exactly in integers
     const double v = 2.0 * cospi((double)q / (2.0 * n));
     const double vi = k == 0 ? 0.5 * v : v;
-    const long long t = (long long)j * n + k;
     buf[off + i] = (T)v;
     buf[off + nn + i] = (T)vi;
-    buf[off + 2 * nn + t] = (T)v;
-    buf[off + 3 * nn + t] = (T)vi;
+    buf[off + 2 * nn + (long long)j * n + k] = (T)vi;
   }
 }
 

@@ -397,7 +397,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
   auto cos_table = [&](int n) {
     auto it = cos_off.find(n);
     if (it != cos_off.end()) return it->second;
-    const long long o = pool.take(4LL * n * n);
+    const long long o = pool.take(3LL * n * n);
     cos_off[n] = o;
     ctx->maxn = std::max(ctx->maxn, n);
     return o;
@@ -596,7 +596,6 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     for (PmlDev& P : ctx->pml) {
       for (int k = 0; k < 3; ++k) P.ap[k] = pool.take(P.n);
       for (int k = 0; k < 2; ++k) { P.aphn[k] = pool.take(P.n); P.apha[k] = pool.take(P.n); P.aphb[k] = pool.take(P.n); }
-      P.aforce = pool.take(3LL * P.A * P.Bp);
     }
     ctx->adj_end = pool.off;
   }

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(128) cube_rows_kernel(CubeArgs<T> a) {
   const DctDev& D = a.dct[q.part];
   const int w = D.w, rows = D.d * D.h;
   const int row0 = (blockIdx.x % a.rows_blocks) * kCubeRows, row = row0 + tid / kCubeLanes;
-  const T* ct = a.buf + D.cw + 3LL * w * w + (long long)(q.x - kCube / 2) * w;
+  const T* ct = a.buf + D.cw + 2LL * w * w + (long long)(q.x - kCube / 2) * w;
   const T* m = a.buf + D.M[a.par] + (long long)min(row, rows - 1) * D.wp;
   if (row0 >= rows) {   // a recorder of a smaller partition than the launch's largest
     grid_dependency_wait();
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(128 * kCubeParts) cube_cols_kernel(CubeArgs<T>
   const int h = D.h, ji = threadIdx.x % 128, part = threadIdx.x / 128;
   const int o = min(ji, kCube * kCube - 1), j = o / kCube, i = o % kCube;
   const T* t1 = a.tmp + (long long)(a.r_lo + rl) * a.s1 + (long long)kz * h * kCube + i;
-  const T* ch = a.buf + D.ch + 3LL * h * h + (long long)(q.y - kCube / 2 + j) * h;
+  const T* ch = a.buf + D.ch + 2LL * h * h + (long long)(q.y - kCube / 2 + j) * h;
   grid_dependency_wait();
   if (kz >= D.d) return;
   const T s = cube_add_parts(cube_part(t1, kCube, ch, h, part));
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(128 * kCubeParts) cube_out_kernel(CubeArgs<T> 
   const DctDev& D = a.dct[q.part];
   const int d = D.d, ji = threadIdx.x % 128, part = threadIdx.x / 128;
   const T* t2 = a.tmp + a.s1 * a.nrec_total + (long long)(a.r_lo + rl) * a.s2 + min(ji, kCube * kCube - 1);
-  const T* cd = a.buf + D.cd + 3LL * d * d + (long long)(q.z - kCube / 2 + k) * d;
+  const T* cd = a.buf + D.cd + 2LL * d * d + (long long)(q.z - kCube / 2 + k) * d;
   grid_dependency_wait();
   const long long t = *a.tcount + a.tstep;
   if (t >= a.max_steps) return;
