@@ -203,9 +203,7 @@ extern "C" int ard_create(const ard_scene* scenes, int32_t n_scenes, const ard_o
     int rc = build_layout(c.get(), scenes, n_scenes);
     if (rc == ARD_OK) rc = configure_kernels(c.get());
     // the GEMM candidate is a distinct layout only where the fused transforms fit
-    if (rc == ARD_OK && cd.gemm &&
-        (c->dct.empty() || c->f2d_bytes > (size_t)std::min(c->smem_optin, 200 * 1024)))
-      rc = ARD_ERR_INVALID;
+    if (rc == ARD_OK && cd.gemm && !c->fused_fit) rc = ARD_ERR_INVALID;
     float ms = 0.f;
     if (rc == ARD_OK) {
       ard_ctx* h = reinterpret_cast<ard_ctx*>(c.get());

@@ -87,6 +87,7 @@ struct Ctx {
   };
   int ngroups = 1;
   AirGroup groups[2];
+  bool fused_fit = false;                  // the fused face transforms' limits are met
   bool fused_faces = false;
   // Tensor-core face transforms (FP32 contexts whose faces take the two-pass
   // form): the four passes as batched split-TF32 products (ard_mma.cuh), with

@@ -212,6 +212,37 @@ bool balance_face_jobs(std::vector<Face2DJob>* jobs, int slots) {
   return split;
 }
 
+// A job whose shared memory leaves one block per SM is split by output.
+static bool one_block_per_sm(const Ctx* ctx, const Face2DJob& J, bool inverse) {
+  const FaceSmem m = face_smem(J, 0, inverse);
+  return (size_t)(m.f + m.a + m.b + m.t) * elem_size(ctx) > 96 * 1024;
+}
+
+static int up4(int v) { return (v + 3) & ~3; }
+
+static FaceSmem widest(const FaceSmem& a, const FaceSmem& b) {
+  return FaceSmem{std::max(a.f, b.f), std::max(a.a, b.a), std::max(a.b, b.b), std::max(a.t, b.t)};
+}
+
+// Bytes of shared memory of the fused face launches of the context's
+// partitions, at most: each region's largest over the jobs before they are
+// balanced (a split job takes no more than the whole one).
+static size_t fused_smem(const Ctx* ctx) {
+  FaceSmem sm{0, 0, 0, 0};
+  auto face = [&](int V, int U) {
+    for (const int ub : {std::min(32, U), U % 32})   // the slabs' widths
+      for (const bool inverse : {false, true}) {
+        if (ub == 0) continue;
+        Face2DJob j{};
+        j.V = V; j.U = U; j.ub = ub;
+        if (one_block_per_sm(ctx, j, inverse)) j.which = 1;
+        sm = widest(sm, face_smem(j, 0, inverse));
+      }
+  };
+  for (const DctDev& D : ctx->dct) { face(D.d, D.h); face(D.d, D.w); face(D.h, D.w); }
+  return (size_t)(up4(sm.f) + up4(sm.a) + up4(sm.b) + up4(sm.t)) * elem_size(ctx);
+}
+
 // Parity-split table `kind` (kFaceC / kFaceCi + kFaceHr / kFaceHf) of extent n.
 static long long face_table(const Ctx* ctx, int n, int kind) {
   for (const auto& kv : ctx->face_tables)
@@ -846,10 +877,15 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     }
   }
 
-  // ---- fused face transforms (one kernel per direction) where a whole layer
-  // pair, both tables' columns and the intermediates fit 200 KB of shared
-  // memory: FP32 extents up to about 132 (larger faces have the rows to feed
-  // the tensor-core passes) ----
+  // ---- fused face transforms (one kernel per direction), for all partitions
+  // of the context or none.  The limit is on extents: V max(U, V) rows of two
+  // whole layers and 32 columns of three operands in 200 KB, 136 cells on every
+  // axis in FP32 and 88 in FP64.  It is the footprint of a full-length kernel;
+  // the quadrants take less, so it leaves faces out that would fit.  At the
+  // limit the fused form is far ahead (GB300, us per step: 40 x 137 x 40 cells
+  // 25 against 68 by the tensor-core passes, FP64 40 x 90 x 40 115 against 502
+  // by the GEMM passes); where the two meet above it is not measured.  What the
+  // launches allocate has to fit as well (fused_smem). ----
   {
     long long xs = 0, bs = 0;
     auto pitch = [](int n) { const int n4 = (n + 3) & ~3; return n4 + ((n4 & 7) ? 8 : 4); };
@@ -858,9 +894,10 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
       bs = std::max(bs, 32LL * (((U + 3) & ~3) + 2 * ((V + 3) & ~3)));
     };
     for (const DctDev& D : ctx->dct) { axis(D.d, D.h); axis(D.d, D.w); axis(D.h, D.w); }
-    ctx->f2d_bytes = (size_t)(2 * xs + bs) * elem_size(ctx);
-    ctx->fused_faces = !ctx->dct.empty() && !ctx->tune_gemm &&
-                       ctx->f2d_bytes <= (size_t)std::min(ctx->smem_optin, 200 * 1024);
+    ctx->fused_fit = !ctx->dct.empty() &&
+                     (size_t)(2 * xs + bs) * elem_size(ctx) <= (size_t)std::min(ctx->smem_optin, 200 * 1024) &&
+                     fused_smem(ctx) <= (size_t)ctx->smem_optin;
+    ctx->fused_faces = ctx->fused_fit && !ctx->tune_gemm;
   }
   if (ctx->fused_faces) {
     std::map<int, long long> tabs;
@@ -1005,8 +1042,7 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     // whole jobs that would leave one block per SM are split by output
     auto presplit = [&](std::vector<Face2DJob>* list, bool inverse) {
       for (size_t i = 0, n = list->size(); i < n; ++i) {
-        const FaceSmem m = face_smem((*list)[i], 0, inverse);
-        if ((size_t)(m.f + m.a + m.b + m.t) * elem_size(ctx) <= 96 * 1024) continue;
+        if (!one_block_per_sm(ctx, (*list)[i], inverse)) continue;
         (*list)[i].which = 1;
         list->push_back((*list)[i]);
         list->back().which = 2;
@@ -1047,15 +1083,13 @@ int build_layout(Ctx* ctx, const ard_scene* scenes, int n_scenes) {
     auto widen = [&](const std::vector<Face2DJob>& list, bool inverse) {
       for (size_t i = 0; i < list.size(); ++i) {
         if (list[i].V == 0) continue;
-        const FaceSmem m = face_smem(list[i], (int)(i & 1), inverse);
-        sm = FaceSmem{std::max(sm.f, m.f), std::max(sm.a, m.a), std::max(sm.b, m.b), std::max(sm.t, m.t)};
+        sm = widest(sm, face_smem(list[i], (int)(i & 1), inverse));
       }
     };
     widen(ctx->fwd2d, false);
     widen(ctx->inv2d, true);
     widen(ctx->adj1_2d, false);
     widen(ctx->adj2_2d, true);
-    auto up4 = [](int v) { return (v + 3) & ~3; };
     ctx->f2d_smem = FaceSmem{up4(sm.f), up4(sm.a), up4(sm.b), up4(sm.t)};
     ctx->f2d_bytes = (size_t)(ctx->f2d_smem.f + ctx->f2d_smem.a + ctx->f2d_smem.b + ctx->f2d_smem.t) * elem_size(ctx);
     if (ctx->f2d_bytes > (size_t)ctx->smem_optin) { ctx->err = "internal: face jobs exceed shared memory"; return ARD_ERR_STATE; }
