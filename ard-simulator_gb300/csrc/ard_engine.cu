@@ -457,11 +457,12 @@ template int launch_pml<double>(Ctx*, int, int, cudaStream_t);
 // Blocks of the partial sums of `total` elements: chunks of 8 elements per thread
 // where the chunks fill a wave of blocks, as many blocks as are resident at
 // once; one element per thread for smaller launches.
-static int sum_launch_blocks(const Ctx* ctx, long long total, bool* chunked) {
+static int sum_launch_blocks(const Ctx* ctx, long long total, int* per) {
   const int wave = ctx->num_sms * 8;
-  *chunked = total / kSumChunk >= wave;
+  const long long nchunks = total / kSumChunk;
+  *per = nchunks >= wave ? 8 : 0;
   if (total <= 0) return 0;
-  return *chunked ? ctx->num_sms * kSumBlocksPerSM : grid_for(total, 256, wave);
+  return *per ? ctx->num_sms * kSumBlocksPerSM : grid_for(total, 256, wave);
 }
 
 // Recorder sums of recorders [r_lo, r_hi) and partial sums of jobs
@@ -471,12 +472,12 @@ int launch_post_modal_range(Ctx* ctx, cudaStream_t s, int tstep, int r_lo, int r
                             long long s_first, long long s_total) {
   const int nrec = r_hi - r_lo;
   const int rec_blocks = (nrec * 32 + 255) / 256;
-  bool chunked;
-  const int sum_blocks = sum_launch_blocks(ctx, s_total, &chunked);
+  int per;
+  const int sum_blocks = sum_launch_blocks(ctx, s_total, &per);
   if (rec_blocks + sum_blocks == 0) return ARD_OK;
   PostModalArgs<T> a{reinterpret_cast<T*>(ctx->d_buf), ctx->d_dct, false, ctx->d_recpts, r_lo, nrec, ctx->n_rec_total,
                      ctx->d_hist, ctx->d_t, tstep, ctx->max_steps, rec_blocks, ctx->d_psum + s_lo, s_hi - s_lo,
-                     s_first, s_total, chunked};
+                     s_first, s_total, per};
   ARD_CUDA(launch_dep(post_modal_kernel<T>, rec_blocks + sum_blocks, 256, 0, s, a));
   ARD_CUDA(cudaGetLastError());
   return ARD_OK;
@@ -490,12 +491,12 @@ template int launch_post_modal_range<double>(Ctx*, cudaStream_t, int, int, int, 
 template <typename T>
 int launch_post_modal_adjoint(Ctx* ctx, cudaStream_t s, const long long* tc, int tstep, double* gsrc) {
   const int n = (int)ctx->srcpts.size(), point_blocks = (n * 32 + 255) / 256;
-  bool chunked;
-  const int sum_blocks = sum_launch_blocks(ctx, ctx->psum_total, &chunked);
+  int per;
+  const int sum_blocks = sum_launch_blocks(ctx, ctx->psum_total, &per);
   if (point_blocks + sum_blocks == 0) return ARD_OK;
   PostModalArgs<T> a{reinterpret_cast<T*>(ctx->d_buf), ctx->d_dct, true, ctx->d_srcpts, 0, n, ctx->n_src_total,
                      gsrc, tc, tstep, ctx->max_steps, point_blocks, ctx->d_psum, (int)ctx->psum.size(),
-                     0, ctx->psum_total, chunked};
+                     0, ctx->psum_total, per};
   ARD_CUDA(launch_dep(post_modal_kernel<T>, point_blocks + sum_blocks, 256, 0, s, a));
   ARD_CUDA(cudaGetLastError());
   return ARD_OK;
