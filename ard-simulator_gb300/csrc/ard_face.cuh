@@ -97,9 +97,9 @@ struct FaceDiv {
 
 // One half-size product per unit: W[u][r][c] = sum_k L[u][r][k] R[u][k][c] for
 // r < rows, c < 4 nq, k < K (a multiple of 4; operands are zero past their
-// extent).  A thread owns MR rows x 4 columns; its rows are rg apart, so the
-// rows that a warp loads together are consecutive.
-template <typename T, int MR, typename LOf, typename ROf, typename Out>
+// extent), from the last k down if REV.  A thread owns MR rows x 4 columns; its
+// rows are rg apart, so the rows that a warp loads together are consecutive.
+template <typename T, bool REV, int MR, typename LOf, typename ROf, typename Out>
 __device__ __forceinline__ void face_product(int units, int rows, int K, const FaceDiv& nq, int lp, int rp, LOf l_of,
                                              ROf r_of, Out out) {
   const FaceDiv rg((rows + MR - 1) / MR);
@@ -115,7 +115,7 @@ __device__ __forceinline__ void face_product(int units, int rows, int K, const F
 #pragma unroll
     for (int i = 0; i < MR; ++i) acc[i][0] = acc[i][1] = {0, 0};
 #pragma unroll 2
-    for (int k = 0; k < K; k += 4) {
+    for (int k = REV ? K - 4 : 0; REV ? k >= 0 : k < K; k += REV ? -4 : 4) {
       T l[MR][4];
       Pair<T> r[4][2];
 #pragma unroll
@@ -123,11 +123,13 @@ __device__ __forceinline__ void face_product(int units, int rows, int K, const F
 #pragma unroll
       for (int i = 0; i < MR; ++i) load4(L + lo[i] + k, l[i]);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
+      for (int q = 0; q < 4; ++q) {
+        const int kk = REV ? 3 - q : q;
 #pragma unroll
         for (int i = 0; i < MR; ++i)
 #pragma unroll
           for (int c = 0; c < 2; ++c) acc[i][c] = fma2(dup2(l[i][kk]), r[kk][c], acc[i][c]);
+      }
     }
 #pragma unroll
     for (int i = 0; i < MR; ++i)
@@ -168,6 +170,16 @@ __device__ __forceinline__ void load_quad(const T* p, int n, bool vec, T (&v)[4]
 // entries of a split job take one parity pu each (INV false) or half of the
 // columns each (INV true).
 //
+// The inverse adds its modes from the highest down (REV).  Its even and odd
+// parts hold the sum and the difference of a cell and its mirror cell, so a quiet
+// cell opposite a loud one gets the rounding of the loud one's sums, where a
+// full-length sum rounds by its own size; with the low modes, the largest, added
+// last, the sums are small until their last terms.  FP32 against FP64, 64 random
+// scenes, recorders over 1200 steps, full-length products / half-length from the
+// low modes up / from the high ones down: geometric mean 3.14e-6 / 3.11e-6 /
+// 3.00e-6, worst (a scene that grows) 7.7e-5 / 1.5e-4 / 7.3e-5.  The order costs
+// no time; sums in blocks of four modes gained nothing more (+4 % in batches).
+//
 // Small launches (one room) are bound by the chain load - product - product -
 // store of one block, large ones (batches) by instruction issue (47 %) and the
 // barriers between the phases.  Layers go through registers once (folded or
@@ -175,8 +187,7 @@ __device__ __forceinline__ void load_quad(const T* p, int n, bool vec, T (&v)[4]
 // split by multiplication (FaceDiv) and the products run on packed FP32 pairs.  GB300, both directions of a step,
 // against full-length products with rows split over a cluster: one 100^3 room
 // 25 -> 17 us, the L-shaped room of 1.9 M cells 51 -> 38 us, 128 scenes 714 ->
-// 435 us (485 us with compiled divisions, 449 us with scalar products); FP64 (0.24 M cells) 213 -> 129 us.  Rounding improves with the
-// shorter sums.
+// 435 us (485 us with compiled divisions, 449 us with scalar products); FP64 (0.24 M cells) 213 -> 129 us.
 template <typename T, bool INV>
 __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ buf, const Face2DJob* __restrict__ jobs,
                                                                int entries, FaceSmem sm) {
@@ -309,8 +320,8 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
     auto b_of = [&](int u) { return Bs + (u & su) * hu4 * ncp; };
     auto to_t = [&](int u, int r, int c, const T (&v)[4]) { store4(Ts + (u * hv4 + r) * ncp + c, v); };
     const bool wide = units * ((hv + 3) >> 2) * nq >= kFaceThreads / 2;
-    if (wide) face_product<T, 4>(units, hv, hu4, dq, fp, ncp, f_of, b_of, to_t);
-    else      face_product<T, 2>(units, hv, hu4, dq, fp, ncp, f_of, b_of, to_t);
+    if (wide) face_product<T, INV, 4>(units, hv, hu4, dq, fp, ncp, f_of, b_of, to_t);
+    else      face_product<T, INV, 2>(units, hv, hu4, dq, fp, ncp, f_of, b_of, to_t);
     __syncthreads();
     if (it + (int)gridDim.x >= entries) grid_launch_dependents();
     // ---- O = A T ----
@@ -327,12 +338,12 @@ __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ b
         for (int e = 0; e < 4; ++e)
           if (c + e < s.nc && ku + 2 * e < U) p[2 * e] = v[e] * scale;
       };
-      if (wide) face_product<T, 4>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_out);
-      else      face_product<T, 2>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_out);
+      if (wide) face_product<T, INV, 4>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_out);
+      else      face_product<T, INV, 2>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_out);
     } else {
       auto to_o = [&](int u, int r, int c, const T (&v)[4]) { store4(Fs + (u * hv + r) * ncp + c, v); };
-      if (wide) face_product<T, 4>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_o);
-      else      face_product<T, 2>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_o);
+      if (wide) face_product<T, INV, 4>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_o);
+      else      face_product<T, INV, 2>(units, hv, hv4, dq, ap, ncp, a_of, t_of, to_o);
       __syncthreads();
       // ---- the quadrants' butterfly ----
       const FaceDiv dc(ncp), dr(hv);
