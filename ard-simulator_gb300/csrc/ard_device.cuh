@@ -44,8 +44,8 @@ constexpr int kMaxPointsPerPart = 8;  // sources or recorders per air partition
 constexpr int kModalWarps = 4;        // warps of a modal tile's block
 constexpr int kModalThreads = 32 * kModalWarps;
 constexpr int kModalTX = 32, kModalTY = 32;   // kx and ky extent of a modal tile
-// Blocks of the modal kernel per SM (FP32: 164 registers, 61 KB of shared memory
-// each; FP64: 255 registers, 112 KB).
+// Blocks of the modal kernel per SM (FP32: 158 registers, 165 in the reference's
+// arithmetic, and 57 KB of shared memory each; FP64: 255 registers, 114 KB).
 template <typename T>
 constexpr int modal_blocks_per_sm() { return sizeof(T) == 4 ? 3 : 2; }
 constexpr int kMaxPmlLayers = 12;

@@ -112,7 +112,7 @@ struct Ctx {
   long long force_begin = 0;                 // all slabs' strip forces: [force_begin, state_end)
   bool adjoint = false;
   // layout choices (the autotuner varies them; defaults are the heuristics)
-  int tune_tiles = 1;      // modal tiles per wave slot (x 2 per SM): kz split finer when > 1
+  int tune_tiles = 1;      // modal tiles per resident slot: kz split finer when > 1
   int tune_gemm = 0;       // 1: two-pass GEMM face transforms even when the fused ones fit
   std::string tuning;      // description of the chosen layout
   // adjoint face transforms (options.adjoint): fused 2D jobs and the two-pass

@@ -181,13 +181,14 @@ __device__ __forceinline__ void load_quad(const T* p, int n, bool vec, T (&v)[4]
 // no time; sums in blocks of four modes gained nothing more (+4 % in batches).
 //
 // Small launches (one room) are bound by the chain load - product - product -
-// store of one block, large ones (batches) by instruction issue (47 %) and the
-// barriers between the phases.  Layers go through registers once (folded or
-// sorted by parity on the way), tables by cp.async underneath; indexes are
-// split by multiplication (FaceDiv) and the products run on packed FP32 pairs.  GB300, both directions of a step,
-// against full-length products with rows split over a cluster: one 100^3 room
-// 25 -> 17 us, the L-shaped room of 1.9 M cells 51 -> 38 us, 128 scenes 714 ->
-// 435 us (485 us with compiled divisions, 449 us with scalar products); FP64 (0.24 M cells) 213 -> 129 us.
+// store of one block, large ones (batches) by the barriers between those phases
+// with two blocks per SM (issue 37 %).  Layers go through registers once (folded
+// or sorted by parity on the way), tables by cp.async underneath; indexes are
+// split by multiplication (FaceDiv) and the products run on packed FP32 pairs.
+// GB300, both directions of a step, against full-length products with rows split
+// over a cluster: one 100^3 room 25 -> 17 us, the L-shaped room of 1.9 M cells
+// 51 -> 38 us, 128 scenes 714 -> 435 us (485 us with compiled divisions, 449 us
+// with scalar products); FP64 (0.24 M cells) 213 -> 129 us.
 template <typename T, bool INV>
 __global__ void __launch_bounds__(kFaceThreads, 2) face_kernel(T* __restrict__ buf, const Face2DJob* __restrict__ jobs,
                                                                int entries, FaceSmem sm) {

@@ -144,8 +144,11 @@ int zero_state(Ctx* ctx) {
 // job), the largest job is split: a two-output job into one job per output,
 // then a one-output job into two halves (face_shape: one parity each, or half
 // of the columns each).  A launch of many waves keeps whole jobs, which read
-// their layers once for all their outputs.  The work model counts whole row
-// blocks of a warp, so a 16-column job weighs as much as a 32-column one.
+// their layers once for all their outputs.  The work model is that of
+// full-length products by whole row blocks of a warp (8 rows of 32 columns, 16
+// of a `narrow` slab's 16): only an order of size for the quadrant kernel, where
+// a slab costs by its quads of columns and the half lengths.  In a split inverse
+// job of at most 8 columns the second entry is empty (face_shape).
 // Output: pairs (jobs[2 i], jobs[2 i + 1]), largest first: a split job twice,
 // or two whole jobs (the last one padded by an empty job).  Returns whether
 // any job is split.

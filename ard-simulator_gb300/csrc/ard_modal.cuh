@@ -73,9 +73,10 @@ constexpr size_t modal_smem_bytes() {
 // and two independent chains cover each other's latency.  GB300, per launch,
 // against one row per thread, cp.async and 256-thread blocks before: 187.5 M
 // cells in 24 partitions with 16 sources and recorders 1.67 -> 0.75 ms (5.0
-// TB/s of the 20 bytes), 48.7 M cells in 128 scenes 604 -> 385 us, 12.4 M
+// TB/s of the 20 bytes), 48.7 M cells in 128 scenes 604 -> 375 us, 12.4 M
 // cells 120 -> 72 us, 1 M cells 18 -> 13 us.  A third stage takes L1 from the
-// other loads (12.4 M cells: 80 against 77 us).  Points cost a launch of
+// other loads (187.5 M cells 737 against 746 us, 128 scenes 378 against 375,
+// rooms equal).  Points cost a launch of
 // their partition 10-20 %; two are handled together to overlap their chains.
 // REF selects the reference's arithmetic.
 //

@@ -21,14 +21,14 @@ advanced one time step; PML cells are extra work, not counted.
           pinned host memory (ard_set_source_samples), the steps, and the
           read-back of that step's recorder samples (ard_read_recorders)
   roofline  the modal kernel (the dominant HBM-bound stage): algorithmic
-          bytes per launch (28 B per air cell, the reference's per-cell
-          reads and writes of one air-partition update) over its CUDA-event
+          bytes per launch (20 B per air cell: two modal levels and two
+          tables read, one level written) over its CUDA-event
           time (ard_profile_steps: the stages of min(steps, 200) un-captured
           steps launched on one stream with events around each), against
           the measured HBM copy bandwidth; traffic = the kernel's DRAM bytes
           per launch from the ncu summary in profiles/
-  stage_roofline  every stage against its bound: PML 44 B per PML cell,
-          interfaces 48 B per face cell, modal 28 B per air cell (HBM), the
+  stage_roofline  every stage against its bound: PML 36 B per PML cell,
+          interfaces 48 B per face cell, modal 20 B per air cell (HBM), the
           face transforms as useful FLOP/s (and, on the tensor-core path, the
           split-TF32 product rate against the dense TF32 rate) and as bytes
           moved against HBM
@@ -76,8 +76,10 @@ sys.path.insert(0, os.path.join(ROOT, "ard-simulator_gb300"))
 
 METRIC = "Gcell-steps/s fwd & fwd+adjoint on 1 GB300 at ≤1e-4 rel recorder err vs FP64"
 UNIT = "Gcell-steps/s"
-BYTES_PER_AIR_CELL = 28      # read f, M, M_prev, cos, psi; write M_next, p (4 B each)
-BYTES_PER_PML_CELL = 44      # read p, p_prev, phi x3, f; write p_next, phi x3, clear f
+BYTES_PER_AIR_CELL = 28      # the reference's: read f, M, M_prev, cos, psi; write M_next, p (4 B each)
+BYTES_PER_PML_CELL = 44      # the reference's: read p, p_prev, phi x3, f; write p_next, phi x3, clear f
+MODAL_BYTES_PER_AIR_CELL = 20   # the kernel's: read M, M_prev and two tables; write M_next (4 B each)
+PML_KERNEL_BYTES_PER_CELL = 36  # the kernel's: read p, p_prev, phi x3; write p_next, phi x3
 BYTES_PER_FACE_CELL = 48     # 6 reads + 6 writes per interface face cell
 MODAL_STAGE = "modal"
 FP32_FMA_TFLOPS = 152 * 128 * 2 * 2.07e9 / 1e12   # CUDA-core FP32 peak at the 2070 MHz maximum SM clock
@@ -623,7 +625,7 @@ def main():
     p_pml = sum(s.pml_cells for s in prof_scenes)
     p_face = sum(s.face_cells for s in prof_scenes)
     modal_ms = stages[MODAL_STAGE]
-    alg_bytes = BYTES_PER_AIR_CELL * p_air
+    alg_bytes = MODAL_BYTES_PER_AIR_CELL * p_air
     achieved = alg_bytes / (modal_ms / 1e3) / 1e9 if modal_ms > 0 else 0.0
     traffic = None
     tpath = os.path.join(ROOT, "profiles", f"traffic_{args.config}.txt")
@@ -655,8 +657,8 @@ def main():
                      "frac_of_fp32_fma_peak": f_tf / FP32_FMA_TFLOPS}
     f_bytes = face_bytes(prof_scenes)
     stage_roofline = {
-        "modal": hbm_stage(modal_ms, BYTES_PER_AIR_CELL * p_air),
-        "pml": hbm_stage(stages["pml"], BYTES_PER_PML_CELL * p_pml),
+        "modal": hbm_stage(modal_ms, alg_bytes),
+        "pml": hbm_stage(stages["pml"], PML_KERNEL_BYTES_PER_CELL * p_pml),
         "iface": hbm_stage(stages["iface"], BYTES_PER_FACE_CELL * p_face),
         "faces": dict({"ms": f_ms, "useful_flops": flops, "achieved_tflops": f_tf,
                        "algorithmic_bytes": f_bytes,
@@ -671,7 +673,8 @@ def main():
                      "achieved": step_bytes / fwd_s_per_time_step / 1e9, "unit": "GB/s",
                      "frac": step_bytes / fwd_s_per_time_step / 1e9 / peak}
     kps = sum(sm.kernels_per_step for sm in sims)
-    launches = int(args.steps * (chunk * kps + (chunk // 32 + (1 if chunk % 32 else 0)) * len(sims)))
+    # a counter launch ends every 32-step graph and every one-step graph of the rest
+    launches = int(args.steps * (chunk * kps + (chunk // 32 + chunk % 32) * len(sims)))
     layout = sim.layout
     for sm in sims:
         sm.close()
