@@ -1,7 +1,9 @@
 """The adjoint's modal update at the edges of its tiles (32 kx x 32 ky x the
 planes of one kz parity) against the FP64 autograd tape: extents just below and
 above a tile, an odd depth (the odd parity one plane short), and up to eight
-sources and recorders, whose injection and read-out change places.
+sources and recorders, whose injection and read-out change places.  The rows are
+padded (no extent along x is a multiple of four), where the reference's arithmetic
+divides by the squared frequency.
 
 Tolerances: the library returns float gradients, so in FP64 their rounding
 (2^-24 of each value; 1e-7 for the series, 1e-6 for the pressure that a dense
@@ -47,8 +49,10 @@ def test_adjoint_modal_tile_edges(extent, points):
     rec = TapeOracle(flat).run(s_t, T, p0={0: p_t})
     target = (0.5 * rec.detach().numpy()[::-1]).astype(np.float32)
     (0.5 * ((rec - torch.tensor(target, dtype=torch.float64)) ** 2).sum()).backward()
-    for precision, tol_s, tol_p in ((A.PREC_F64, 1e-7, 1e-6), (A.PREC_F32, 2.9e-5, 2.9e-5)):
-        sim = A.Simulation(A.scene_from_flat(flat), precision=precision, max_steps=T, adjoint=True)
+    for precision, arithmetic, tol_s, tol_p in ((A.PREC_F64, A.ARITH_ACCURATE, 1e-7, 1e-6),
+                                                (A.PREC_F64, A.ARITH_REFERENCE, 1e-7, 1e-6),
+                                                (A.PREC_F32, A.ARITH_ACCURATE, 2.9e-5, 2.9e-5)):
+        sim = A.Simulation(A.scene_from_flat(flat), precision=precision, arithmetic=arithmetic, max_steps=T, adjoint=True)
         for i, s in enumerate(series):
             sim.set_source_series(i, s)
         sim.set_initial_pressure(0, p0)
