@@ -577,7 +577,13 @@ static int launch_single_steps(Ctx* ctx, int n, cudaStream_t s) {
   }
   for (int i = d; i < n; ++i) {
     const int par = (int)(ctx->t_host & 1);
-    if (int rc = capture_steps(ctx, 1, par, &ctx->step_exec[par])) return rc;
+    if (capture_steps(ctx, 1, par, &ctx->step_exec[par]) != ARD_OK) {
+      // no graph (a full device has no memory for one): direct launches need
+      // none, and report what they cannot do themselves
+      cudaGetLastError();
+      ctx->err.clear();
+      return launch_steps_direct(ctx, n - i, s);
+    }
     ARD_CUDA(cudaGraphLaunch(ctx->step_exec[par], s));
     ++ctx->t_host;
   }
